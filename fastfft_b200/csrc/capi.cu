@@ -37,14 +37,16 @@ using namespace ffb;
 #define FFB_XCORR_TPB 8
 #endif
 
-// templates that one block of the fused column pass stages for a launch of n at column
-// length my; measured best on B200 with 64 per launch: six at 1536 (= 3 * 512; 5.37 instead of
-// 5.47 us per template for that pass; 4, 5 and 8 were slower), four at 1024 (1.99 instead of
-// 2.06; 6 and 16 were slower), eight elsewhere (at 256: 0.23 against 0.29 with four)
+// templates that one block of the fused column pass serves for a launch of n at column length
+// my; measured best on B200: at 1536 twelve from 16 templates up (266 us per 64-template launch;
+// 282 - 300 with the tensor-core and three-group forms' 6) and six below, at 384 four up to 16
+// templates (10.0 instead of 14.3 us at 12) and eight above, eight elsewhere (at 1024: 66.1 us
+// per 32 templates; 68.7 with four or six, 70.6 with twelve)
 // (fastfft_set_templates_per_block overrides it; the autotuner measures the candidates)
 static inline int xcorr_tpb(const fastfft_plan_s* h, int n, long long my) {
     const int per_block = h->tpb_request > 0 ? h->tpb_request
-                          : FFB_XCORR_TPB != 8 ? FFB_XCORR_TPB : my == 3 * 512 ? 6 : my == 1024 ? 4 : 8;
+                          : FFB_XCORR_TPB != 8 ? FFB_XCORR_TPB
+                          : my == 3 * 512 ? (n >= 16 && !h->tc_dft ? 12 : 6) : my == 384 && n <= 16 ? 4 : 8;
     return per_block > 0 && n > per_block ? per_block : n;
 }
 

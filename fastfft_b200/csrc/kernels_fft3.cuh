@@ -359,7 +359,7 @@ struct Xcorr3Smem {
 };
 
 
-template <int R, int P, class ImgC, int FPB, bool MUL>
+template <int R, int P, class ImgC, int FPB>
 __global__ void __launch_bounds__(FftRShape<R, P>::T * FPB,
                                   FftRShape<R, P>::T * FPB < kXcorr3SmThreads ? kXcorr3SmThreads / (FftRShape<R, P>::T * FPB) : 1)
 xcorr3_cols_kernel(XcorrColArgs a) {
@@ -440,17 +440,15 @@ xcorr3_cols_kernel(XcorrColArgs a) {
             }
         }
         BlockFft<P, false>::run(v, grp, j, a.tw, live ? leading_slots_p<P>(Lg, j) : 0);
-        if constexpr (MUL) {
-            // CONJ_MUL (scale 1) skips the 32 multiplies of the scaling
-            if (sc == 1.f) {
+        // CONJ_MUL (scale 1) skips the 32 multiplies of the scaling
+        if (sc == 1.f) {
 #pragma unroll
-                for (int q = 0; q < 16; q++) v[q] = conj_mul(v[q], lds_cplx<ImgC>(img_s + R * (j + TP * q) + k2));
-            } else {
+            for (int q = 0; q < 16; q++) v[q] = conj_mul(v[q], lds_cplx<ImgC>(img_s + R * (j + TP * q) + k2));
+        } else {
 #pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const float2 im = lds_cplx<ImgC>(img_s + R * (j + TP * q) + k2);
-                    v[q] = cscale(conj_mul(v[q], im), sc);
-                }
+            for (int q = 0; q < 16; q++) {
+                const float2 im = lds_cplx<ImgC>(img_s + R * (j + TP * q) + k2);
+                v[q] = cscale(conj_mul(v[q], im), sc);
             }
         }
         BlockFft<P, true>::run(v, grp, j, a.tw, 16);

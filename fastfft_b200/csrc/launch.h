@@ -28,6 +28,8 @@ cudaError_t launch_cols_xcorr(int n, int img_dtype, const ColArgs& a, cudaStream
 // Batched fused column pass (TMA-staged image and template columns), n <= 4096.
 cudaError_t launch_xcorr_cols(int n, int img_dtype, const XcorrColArgs& a, cudaStream_t st);
 size_t xcorr_cols_smem(int n, int img_dtype, int L, int n_batch);
+// The same pass on the split block FFT (fft_split.cuh), which launch_xcorr_cols takes at its lengths.
+cudaError_t launch_xcorr_split(int n, const XcorrColArgs& a, cudaStream_t st);
 
 // Lengths N = 3P (128 <= P <= 2048): the reduced-size correlation's internal sizes and the
 // 2D plans at these sizes; the public launchers above forward them here.
@@ -62,6 +64,8 @@ cudaError_t launch_radial_power(const RadialArgs& a, float* power, cudaStream_t 
 // Device-wide FP64-generated twiddle tables (generated once per device): for a power of
 // two n the radix-16 pass table, for n = 3P the radix-3 pass table W_n^m, m < 2P.
 cudaError_t twiddles_for(int n, const float2** out);
+// ... and the split block FFT's table of length n (fft_split.cuh).
+cudaError_t split_twiddles_for(int n, const float2** out);
 
 // Message returned by fastfft_last_error(NULL), for entry points without a handle.
 void set_unbound_error(const char* msg);

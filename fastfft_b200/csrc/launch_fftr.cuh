@@ -207,6 +207,9 @@ constexpr int kMaxDynSmem3 = 227 * 1024 - 1024;
 
 template <int R, int P, class ImgC>
 static cudaError_t xcorr3_impl(const XcorrColArgs& a0, cudaStream_t st) {
+    if constexpr (is_split_size(R * P)) {
+        return launch_xcorr_split(R * P, a0, st);
+    } else {
     constexpr int FPB = xcorr3_fpb<R, P>();
     using SM = Xcorr3Smem<R, P, ImgC, FPB>;
     if (a0.n_batch < 1 || a0.n_batch > kMaxBatch || a0.n_cols < 1) return cudaErrorInvalidValue;
@@ -216,22 +219,17 @@ static cudaError_t xcorr3_impl(const XcorrColArgs& a0, cudaStream_t st) {
     XcorrColArgs a = a0;
     cudaError_t e = tables3(R, P, &a.tw, &a.tw3);
     if (e != cudaSuccess) return e;
-    static std::atomic<int> set_attr[2][64];
-    const bool mul = a.intra_kind != 0;
-    auto fn = mul ? xcorr3_cols_kernel<R, P, ImgC, FPB, true> : xcorr3_cols_kernel<R, P, ImgC, FPB, false>;
-    if ((e = ensure_smem_at_least((const void*)fn, (size_t)smem, set_attr[mul])) != cudaSuccess) return e;
+    static std::atomic<int> high_water[64];
+    auto fn = xcorr3_cols_kernel<R, P, ImgC, FPB>;
+    if ((e = ensure_smem_at_least((const void*)fn, (size_t)smem, high_water)) != cudaSuccess) return e;
     fn<<<dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), FftRShape<R, P>::T * FPB, smem, st>>>(a);
     return cudaGetLastError();
+    }
 }
 
 template <int R, int P>
 static cudaError_t xcorr3_dispatch(int img_dtype, const XcorrColArgs& a, cudaStream_t st) {
-    switch (img_dtype) {
-        case 3: return xcorr3_impl<R, P, float2>(a, st);
-        case 4: return xcorr3_impl<R, P, __half2>(a, st);
-        case 5: return xcorr3_impl<R, P, __nv_bfloat162>(a, st);
-        default: return cudaErrorInvalidValue;
-    }
+    return img_dtype == 3 ? xcorr3_impl<R, P, float2>(a, st) : cudaErrorInvalidValue;
 }
 
 template <int R>

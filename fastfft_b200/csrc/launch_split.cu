@@ -1,0 +1,66 @@
+// Launcher of the batched fused correlation column pass on the split block FFT
+// (xcorr_split_kernel in kernels_xcorr.cuh).
+#include "kernels_xcorr.cuh"
+#include "launch_common.cuh"
+
+namespace ffb {
+
+template <int N, class C, int G, int MIN_BLOCKS>
+static cudaError_t xcorr_split_impl(const XcorrColArgs& a, cudaStream_t st) {
+    const int smem = XcorrSplitSmem<N, C, G>::total(a.L);
+    static std::atomic<int> high_water[64];
+    auto fn = xcorr_split_kernel<N, C, G, MIN_BLOCKS>;
+    cudaError_t e = ensure_smem_at_least((const void*)fn, (size_t)smem, high_water);
+    if (e != cudaSuccess) return e;
+    fn<<<dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), SplitFft<N, C>::T * G, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+// Blocks of G transform groups; registers for MIN_BLOCKS blocks per SM.  Measured on B200 (us per
+// launch; "before": the radix-16 forms xcorr_cols_kernel / xcorr3_cols_kernel, which keep the
+// other lengths):
+//   length (template, window, templates)   before   single value   pair
+//   1536 (384, 1024, 64)                     333    288 (2 x 4)    266 (2 x 3), 284 (3 x 2)
+//   1536 (384, 1024, 12)                      85     65 (2 x 4)     67 (3 x 2)
+//   1536 (384, 1024, 1)                     17.2   13.9 (1 x 8)   18.3 (1 x 6)
+//   768  (256, 512, 64)                       90     80 (4 x 4)     80 (4 x 3)
+//   384  (96, 256, 64)                      34.2   25.5 (4 x 8)   26.4 (4 x 6)
+//   1024 (384, 512, 32)                     69.6   66.1 (2 x 4)   70.3 (2 x 3)
+//   512  (150, 300, 32)                     25.4   20.6 (4 x 4)   23.4 (4 x 3)
+//   256  (60, 128, 32)                      12.0    9.7 (8 x 5)    9.9 (8 x 3)
+//   2048 (500, 1100, 16)                     159    136 (1 x 4)    129 (1 x 3)
+// The single form at 128 registers (16 warps per SM) is the better one at most lengths (at 96 it
+// spills: 382 us at 1536); at 2048, and at 1536 once a launch holds 16 templates, the pair is (168
+// registers, 12 warps).  Fewer than four templates take blocks of one group, so that no group
+// idles.  At 1536 the pair's launch keeps the FP32 pipe 53 %, the shared-memory path 65 % and the
+// issue slots 57 % busy at 3 warps per scheduler: bound by latency at that occupancy (before: 48,
+// 75 and 71 %).  Both forms give the same bits (cpair.cuh), so the choice does not show in results.
+cudaError_t launch_xcorr_split(int n, const XcorrColArgs& a0, cudaStream_t st) {
+    XcorrColArgs a = a0;
+    if (a.n_batch < 1 || a.n_batch > kMaxBatch || a.n_cols < 1 || a.L < 1 || a.L > n) return cudaErrorInvalidValue;
+    if (a.tpb < 1 || a.tpb > a.n_batch) return cudaErrorInvalidValue;
+    cudaError_t e = split_twiddles_for(n, &a.tw);
+    if (e != cudaSuccess) return e;
+    const bool few = a.n_batch < 4;
+    switch (n) {
+        case 256: return xcorr_split_impl<256, float2, 8, 5>(a, st);
+        case 384: return xcorr_split_impl<384, float2, 4, 8>(a, st);
+        case 512: return xcorr_split_impl<512, float2, 4, 4>(a, st);
+        case 768:
+            if (few) return xcorr_split_impl<768, float2, 1, 16>(a, st);
+            return xcorr_split_impl<768, float2, 4, 4>(a, st);
+        case 1024:
+            if (few) return xcorr_split_impl<1024, float2, 1, 8>(a, st);
+            return xcorr_split_impl<1024, float2, 2, 4>(a, st);
+        case 1536:
+            if (few) return xcorr_split_impl<1536, float2, 1, 8>(a, st);
+            if (a.n_batch < 16) return xcorr_split_impl<1536, float2, 2, 4>(a, st);
+            return xcorr_split_impl<1536, cpair, 2, 3>(a, st);
+        case 2048:
+            if (few) return xcorr_split_impl<2048, float2, 1, 4>(a, st);
+            return xcorr_split_impl<2048, cpair, 1, 3>(a, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace ffb

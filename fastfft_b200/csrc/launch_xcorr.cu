@@ -16,6 +16,8 @@ template <int N, class ImgC>
 static cudaError_t xcorr_v2_impl(const XcorrColArgs& a, cudaStream_t st) {
     if constexpr (N > 4096) {
         return cudaErrorInvalidValue;
+    } else if constexpr (is_split_size(N)) {
+        return launch_xcorr_split(N, a, st);
     } else {
         constexpr int FPB = xcorr_fpb<N>();
         using SM = XcorrSmem<N, ImgC, FPB>;
@@ -23,10 +25,9 @@ static cudaError_t xcorr_v2_impl(const XcorrColArgs& a, cudaStream_t st) {
         if (a.tpb < 1 || a.tpb > a.n_batch) return cudaErrorInvalidValue;
         const int smem = SM::total(a.L, a.tpb);
         if (smem > kMaxDynSmem) return cudaErrorInvalidValue;
-        static std::atomic<int> set_mul[64], set_nomul[64];
-        const bool mul = a.intra_kind != 0;
-        auto fn = mul ? xcorr_cols_kernel<N, ImgC, FPB, true> : xcorr_cols_kernel<N, ImgC, FPB, false>;
-        cudaError_t e = ensure_smem_at_least((const void*)fn, (size_t)smem, mul ? set_mul : set_nomul);
+        static std::atomic<int> high_water[64];
+        auto fn = xcorr_cols_kernel<N, ImgC, FPB>;
+        cudaError_t e = ensure_smem_at_least((const void*)fn, (size_t)smem, high_water);
         if (e != cudaSuccess) return e;
         fn<<<dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), FftShape<N>::T * FPB, smem, st>>>(a);
         return cudaGetLastError();
@@ -35,15 +36,12 @@ static cudaError_t xcorr_v2_impl(const XcorrColArgs& a, cudaStream_t st) {
 
 template <int N>
 static cudaError_t xcorr_v2_dispatch(int img_dtype, const XcorrColArgs& a, cudaStream_t st) {
-    switch (img_dtype) {
-        case 3: return xcorr_v2_impl<N, float2>(a, st);
-        case 4: return xcorr_v2_impl<N, __half2>(a, st);
-        case 5: return xcorr_v2_impl<N, __nv_bfloat162>(a, st);
-        default: return cudaErrorInvalidValue;
-    }
+    // the prepared image spectrum is FP32 whatever the image's storage
+    return img_dtype == 3 ? xcorr_v2_impl<N, float2>(a, st) : cudaErrorInvalidValue;
 }
 
 cudaError_t launch_xcorr_cols(int n, int img_dtype, const XcorrColArgs& a, cudaStream_t st) {
+    if (a.intra_kind != 2 && a.intra_kind != 3) return cudaErrorInvalidValue;
     if (is_rp_size(n)) return launch_xcorr3(n, img_dtype, a, st);
     FFB_SIZE_SWITCH(n, xcorr_v2_dispatch, img_dtype, a, st)
 }

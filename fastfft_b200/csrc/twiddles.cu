@@ -1,6 +1,7 @@
 // Device-wide twiddle table and per-device/per-kernel one-time set-up.
 #include <mutex>
 
+#include "fft_split.cuh"
 #include "launch_common.cuh"
 
 namespace ffb {
@@ -70,6 +71,25 @@ static __global__ void init_twiddles_r_kernel(float2* tw, int r) {
     }
 }
 
+// Tables of the split block FFT (layout at tws_size_of in fft_split.cuh).
+static __global__ void init_twiddles_split_kernel(float2* tw) {
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= kTwsTotal) return;
+    int base = 0, n = 0;
+    for (int i = 0; i < kSplitCount; i++) {
+        n = split_size(i);
+        if (gid < base + tws_size_of(n)) break;
+        base += tws_size_of(n);
+    }
+    const int local = gid - base, p = n / split_e(n), b = split_b(n);
+    // W_n^(s j), then W_p^(k1 i)
+    const double x = local < n ? -2.0 * ((double)(local / p) * (local % p)) / n
+                               : -2.0 * ((double)((local - n) / b) * ((local - n) % b)) / p;
+    double sv, cv;
+    sincospi(x, &sv, &cv);
+    tw[gid] = make_float2((float)cv, (float)sv);
+}
+
 // One table for every supported size, generated on the device in FP64 and rounded
 // once to FP32 (the reference evaluates __sincosf per element instead,
 // include/detail/device_functions.h:17-27).
@@ -77,6 +97,7 @@ __device__ float2 g_twiddles[kTwTotal];
 __device__ float2 g_twiddles3[kTw3Total];
 __device__ float2 g_twiddles5[kTw5Total];
 __device__ float2 g_twiddles7[kTw7Total];
+__device__ float2 g_twiddles_split[kTwsTotal];
 
 namespace {
 std::mutex g_tw_mutex;
@@ -84,6 +105,7 @@ const float2* g_tw_ptr[64] = {nullptr};
 const float2* g_tw3_ptr[64] = {nullptr};
 const float2* g_tw5_ptr[64] = {nullptr};
 const float2* g_tw7_ptr[64] = {nullptr};
+const float2* g_tws_ptr[64] = {nullptr};
 }  // namespace
 
 cudaError_t twiddles_for(int n, const float2** out) {
@@ -97,6 +119,7 @@ cudaError_t twiddles_for(int n, const float2** out) {
         void* p3 = nullptr;
         void* p5 = nullptr;
         void* p7 = nullptr;
+        void* ps = nullptr;
         e = cudaGetSymbolAddress(&p, g_twiddles);
         if (e != cudaSuccess) return e;
         e = cudaGetSymbolAddress(&p3, g_twiddles3);
@@ -104,6 +127,8 @@ cudaError_t twiddles_for(int n, const float2** out) {
         e = cudaGetSymbolAddress(&p5, g_twiddles5);
         if (e != cudaSuccess) return e;
         e = cudaGetSymbolAddress(&p7, g_twiddles7);
+        if (e != cudaSuccess) return e;
+        e = cudaGetSymbolAddress(&ps, g_twiddles_split);
         if (e != cudaSuccess) return e;
         cudaStream_t s;
         e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
@@ -122,6 +147,10 @@ cudaError_t twiddles_for(int n, const float2** out) {
             init_twiddles_r_kernel<<<(kTw7Total + 255) / 256, 256, 0, s>>>(static_cast<float2*>(p7), 7);
             e = cudaGetLastError();
         }
+        if (e == cudaSuccess) {
+            init_twiddles_split_kernel<<<(kTwsTotal + 255) / 256, 256, 0, s>>>(static_cast<float2*>(ps));
+            e = cudaGetLastError();
+        }
         cudaError_t e2 = cudaStreamSynchronize(s);
         cudaStreamDestroy(s);
         if (e != cudaSuccess) return e;
@@ -130,6 +159,7 @@ cudaError_t twiddles_for(int n, const float2** out) {
         g_tw3_ptr[dev] = static_cast<const float2*>(p3);
         g_tw5_ptr[dev] = static_cast<const float2*>(p5);
         g_tw7_ptr[dev] = static_cast<const float2*>(p7);
+        g_tws_ptr[dev] = static_cast<const float2*>(ps);
     }
     if (is_3p_size(n)) {
         *out = g_tw3_ptr[dev] + twr_base(3, n / 3);
@@ -148,6 +178,17 @@ cudaError_t twiddles_for(int n, const float2** out) {
     int base = 0;
     for (int m = kMinN; m < n; m *= 2) base += tw_size_of(m);
     *out = g_tw_ptr[dev] + base;
+    return cudaSuccess;
+}
+
+cudaError_t split_twiddles_for(int n, const float2** out) {
+    if (!is_split_size(n)) return cudaErrorInvalidValue;
+    const float2* any = nullptr;
+    cudaError_t e = twiddles_for(n, &any);   // generates every table of the device on first use
+    if (e != cudaSuccess) return e;
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    *out = g_tws_ptr[dev] + tws_base(n);
     return cudaSuccess;
 }
 

@@ -396,17 +396,17 @@ __device__ __forceinline__ void twiddle_pass(float2 (&v)[16], float2 w1, float2 
 }
 
 // Exchange buffers and barrier of one FFT group (T = N/16 threads) inside a block of
-// FPB groups.  Groups of at least one warp synchronise on their own named barrier
-// (bar.sync 1 + f, T), so the groups of a block do not wait for each other; smaller
-// groups fall back to __syncthreads().  With DB (double buffering) consecutive
+// FPB groups.  Groups of up to one warp (which lie within a warp) synchronise with
+// __syncwarp(), larger ones on their own named barrier (bar.sync 1 + f, T), so the groups
+// of a block do not wait for each other.  With DB (double buffering) consecutive
 // exchanges alternate between two buffers, which makes the write-after-read barrier
 // unnecessary: a buffer is rewritten only after a barrier that every thread reaches
-// after its last read of it.
-template <int N, int FPB, bool DB>
+// after its last read of it.  PAD: float2 per buffer.
+template <int N, int FPB, bool DB, int PAD = FftShape<N>::SMEM_PAD>
 struct FftGroup {
     using S = FftShape<N>;
     static constexpr int T = S::T;
-    static constexpr int STRIDE = (DB ? 2 : 1) * S::SMEM_PAD;  // float2 per group
+    static constexpr int STRIDE = (DB ? 2 : 1) * PAD;  // float2 per group
     static constexpr int BYTES = FPB * STRIDE * (int)sizeof(float2);  // per block
     float2* base;
     int f;
@@ -415,7 +415,9 @@ struct FftGroup {
     __device__ __forceinline__ FftGroup(float2* smem_block, int group) : base(smem_block + group * STRIDE), f(group), k(0) {}
 
     __device__ __forceinline__ void sync() const {
-        if constexpr (T >= 32 && FPB > 1 && FPB <= 15) {
+        if constexpr (T <= 32) {
+            __syncwarp();
+        } else if constexpr (FPB > 1 && FPB <= 15) {
             asm volatile("bar.sync %0, %1;" ::"r"(f + 1), "n"(T) : "memory");
         } else {
             __syncthreads();
@@ -426,7 +428,7 @@ struct FftGroup {
     __device__ __forceinline__ float2* begin() {
         float2* p = base;
         if constexpr (DB) {
-            p += (k & 1) * S::SMEM_PAD;
+            p += (k & 1) * PAD;
         } else {
             sync();
         }
@@ -446,7 +448,7 @@ struct BlockFft {
     // X[j + T q], q < qout, the caller keeps (16 = all); the last pass computes only those
     // where the pass structure allows it (the others are left undefined).  Every thread of
     // the group must call this (and, for groups smaller than a warp, every thread of the
-    // block).
+    // warp).
     template <class G>
     __device__ __forceinline__ static void run(float2 (&v)[16], G& g, int j, const float2* __restrict__ tw, int qnz,
                                                int qout = 16) {

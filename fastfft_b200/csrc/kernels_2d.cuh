@@ -250,11 +250,26 @@ struct ColArgs {
     int out_coalesce;
 };
 
+// Exchange groups of cols_kernel.  Blocks of several columns (N < 4096) in the plain forward and
+// inverse modes keep one buffer per column and registers for four 256-thread blocks per SM: these
+// passes wait for memory, and 32 warps per SM cover that better than the 16 that double
+// buffering and 128 registers left (the correlation, with two transforms per column, keeps
+// those).  The stride of the buffers puts the columns that a half-warp of the coalesced store
+// reads (FPB of them at each element) into different banks; at 4 modulo 16 the 256-point passes
+// read four columns per bank.
+template <int N, int MODE, int FPB>
+struct ColGroup {
+    static constexpr bool kMany = FPB > 1 && MODE != COL_XCORR;
+    static constexpr int kPad = (FftShape<N>::SMEM + 15) / 16 * 16 + (FPB >= 16 ? 1 : FPB > 1 ? 16 / FPB : 4);
+    static constexpr int kMinBlocks = FftShape<N>::T * FPB > 256 ? 1 : kMany ? 4 : 2;
+    using G = FftGroup<N, FPB, !kMany, kPad>;
+};
+
 // Shared-memory plan of cols_kernel (bytes): the FFT groups' exchange buffers, then (when the
 // image column is staged) the column and its barrier.
-template <int N, class ImgC, int FPB>
+template <int N, int MODE, class ImgC, int FPB>
 struct ColSmem {
-    static constexpr int kXchBytes = FftGroup<N, FPB, true>::BYTES;
+    static constexpr int kXchBytes = ColGroup<N, MODE, FPB>::G::BYTES;
     static constexpr int kImgOff = (kXchBytes + 127) & ~127;
     static constexpr int kImgBytes = N * (int)sizeof(ImgC);
     static constexpr int kBarOff = (kImgOff + kImgBytes + 15) & ~15;
@@ -262,13 +277,13 @@ struct ColSmem {
 };
 
 template <int N, int MODE, class InC, class ImgC, class OutC, int FPB>
-__global__ void __launch_bounds__(FftShape<N>::T * FPB, (FftShape<N>::T * FPB <= 256) ? 2 : 1)
+__global__ void __launch_bounds__(FftShape<N>::T * FPB, ColGroup<N, MODE, FPB>::kMinBlocks)
 cols_kernel(ColArgs a) {
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ __align__(128) float2 smem[];
-    using G = FftGroup<N, FPB, true>;
-    using CS = ColSmem<N, ImgC, FPB>;
+    using G = typename ColGroup<N, MODE, FPB>::G;
+    using CS = ColSmem<N, MODE, ImgC, FPB>;
     const int f = threadIdx.x / T;
     const int j = threadIdx.x - f * T;
     G g(smem, f);

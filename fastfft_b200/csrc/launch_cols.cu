@@ -7,7 +7,7 @@ template <int N, int MODE, class ImgC, class InC = float2, class OutC = float2>
 static cudaError_t cols_impl(const ColArgs& args, cudaStream_t st) {
     constexpr int FPB = col_fpb<N>();
     constexpr int THREADS = FftShape<N>::T * FPB;
-    using CS = ColSmem<N, ImgC, FPB>;
+    using CS = ColSmem<N, MODE, ImgC, FPB>;
     ColArgs a = args;
     // The fused pass with one column per block stages its image column by a bulk copy when
     // every column starts on a 16-byte boundary (cp.async.bulk needs 16-byte aligned

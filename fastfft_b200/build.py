@@ -15,7 +15,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "_build"
 LIB = PKG / "libfastfft_b200.so"
-SOURCES = ["launch_fft7.cu", "launch_fft5.cu", "launch_fft3.cu", "twiddles.cu", "launch_rows.cu", "launch_cols.cu", "launch_xcorr.cu", "launch_split.cu",
+SOURCES = ["launch_blue_8k.cu", "launch_blue_4k.cu", "launch_blue_2k.cu", "launch_fft7.cu", "launch_fft5.cu", "launch_fft3.cu", "twiddles.cu", "launch_rows.cu", "launch_cols.cu", "launch_xcorr.cu", "launch_split.cu",
            "capi.cu", "noalloc.cu", "spectrum_ops.cu", "launch_tc.cu", "launch_blue.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

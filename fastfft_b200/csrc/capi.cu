@@ -489,7 +489,6 @@ ColArgs col_args(const void* in, long long in_stride, int L, void* out, long lon
     c.out_stride = out_stride;
     c.W = W;
     c.n_cols = n_cols;
-    c.in_scale = 1.f;
     c.out_scale = 1.f;
     c.intra_scale = 1.f;
     c.n_batch = 1;

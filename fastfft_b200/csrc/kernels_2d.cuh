@@ -160,15 +160,15 @@ r2c_rows_kernel(RowFwdArgs a) {
     const InT* pb = in_g + input_row(ra + 1, a.rows_y, a.rows_z) * in_pitch;
     float2* const out_g = a.out + (long long)gb * a.out_batch_stride;
     float2 v[16];
+    const int La = has_a ? L : 0, Lb = has_b ? L : 0;
 #pragma unroll
     for (int q = 0; q < 16; q++) {
         const int n = j + T * q;
-        float xa = 0.f, xb = 0.f;
-        if (n < L) {
-            if (has_a) xa = ld_real<InT>(pa + n);
-            if (has_b) xb = ld_real<InT>(pb + n);
-        }
-        v[q] = make_float2(xa * a.scale, xb * a.scale);
+        v[q] = make_float2(n < La ? ld_real<InT>(pa + n) : 0.f, n < Lb ? ld_real<InT>(pb + n) : 0.f);
+    }
+    if (a.scale != 1.f) {
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = cscale(v[q], a.scale);
     }
     BlockFft<N, false>::run(v, g, j, a.tw, leading_slots<T>(L, j));
 
@@ -223,7 +223,6 @@ struct ColArgs {
     int n_cols;
     int intra_kind;          // 0 NOOP, 2 CONJ_MUL, 3 CONJ_MUL_THEN_SCALE
     float intra_scale;
-    float in_scale;
     float out_scale;
     const float2* tw;
     const float2* tw3;       // N = 3P: radix-3 pass twiddles (set by the launcher)
@@ -312,14 +311,10 @@ cols_kernel(ColArgs a) {
     const InC* pin = static_cast<const InC*>(a.in) + bz * a.in_batch_stride + (long long)(col / in_div) * a.in_stride +
                      (long long)(col % in_div) * a.in_stride2;
     float2 v[16];
+    const int Lc = valid ? a.L : 0;
 #pragma unroll
-    for (int q = 0; q < 16; q++) {
-        const int n = j + T * q;
-        float2 x = make_float2(0.f, 0.f);
-        if (valid && n < a.L) x = ld_cplx<InC>(pin + n);
-        v[q] = (a.in_scale != 1.f) ? cscale(x, a.in_scale) : x;
-    }
-    const int qnz = valid ? leading_slots<T>(a.L, j) : 0;
+    for (int q = 0; q < 16; q++) v[q] = j + T * q < Lc ? ld_cplx<InC>(pin + j + T * q) : make_float2(0.f, 0.f);
+    const int qnz = leading_slots<T>(Lc, j);
     // output pruning: a window at the origin keeps X[j + T q] for q < qout only
     const int qout = a.W0 == 0 ? leading_slots<T>(a.W, j) : 16;
     if constexpr (MODE == COL_INV) {
@@ -344,27 +339,28 @@ cols_kernel(ColArgs a) {
             __syncthreads();
             if (!img_ok) return;
             mbar_wait(img_bar, 0);
-            const float sc = a.intra_kind == 3 ? a.intra_scale : 1.f;
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const float2 p = conj_mul(v[q], lds_cplx<ImgC>(img_s + j + T * q));
-                v[q] = (sc != 1.f) ? cscale(p, sc) : p;
-            }
+            for (int q = 0; q < 16; q++) v[q] = conj_mul(v[q], lds_cplx<ImgC>(img_s + j + T * q));
         } else if (a.intra_kind != 0) {
             const ImgC* pimg = static_cast<const ImgC*>(a.img) + bz * a.img_batch_stride + (long long)col * a.img_stride;
-            const float sc = a.intra_kind == 3 ? a.intra_scale : 1.f;
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                float2 im = make_float2(0.f, 0.f);
-                if (valid) im = ld_cplx_stream<ImgC>(pimg + j + T * q);
-                float2 p = conj_mul(v[q], im);
-                v[q] = (sc != 1.f) ? cscale(p, sc) : p;
-            }
+            for (int q = 0; q < 16; q++)
+                v[q] = conj_mul(v[q], valid ? ld_cplx_stream<ImgC>(pimg + j + T * q) : make_float2(0.f, 0.f));
+        }
+        if (a.intra_kind == 3 && a.intra_scale != 1.f) {
+#pragma unroll
+            for (int q = 0; q < 16; q++) v[q] = cscale(v[q], a.intra_scale);
         }
         BlockFft<N, true>::run(v, g, j, a.tw, 16, qout);
     }
     const int out_div = a.out_div > 0 ? a.out_div : 1;
     const long long es = a.out_elem_stride > 0 ? a.out_elem_stride : 1;
+    // (scales and offsets that a call does not use are tested once, outside the element loops:
+    // per element they were a quarter of this kernel's instructions at 4096 points)
+    if (a.out_scale != 1.f) {
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = cscale(v[q], a.out_scale);
+    }
     if constexpr (FPB > 1) {
         if (a.out_coalesce) {
             // every group parks its column in its own buffer (natural order), then item i of
@@ -379,10 +375,7 @@ cols_kernel(ColArgs a) {
                           (long long)(c0 / out_div) * a.out_stride + (long long)(c0 % out_div) * a.out_stride2;
             for (int i = threadIdx.x; i < a.W * FPB; i += T * FPB) {
                 const int n = i / FPB, ff = i - n * FPB;
-                if (ff < cols_here) {
-                    const float2 x = smem[ff * G::STRIDE + phys(n + a.W0)];
-                    st_cplx<OutC>(pout0 + ff + n * es, (a.out_scale != 1.f) ? cscale(x, a.out_scale) : x);
-                }
+                if (ff < cols_here) st_cplx<OutC>(pout0 + ff + n * es, smem[ff * G::STRIDE + phys(n + a.W0)]);
             }
             return;
         }
@@ -390,12 +383,15 @@ cols_kernel(ColArgs a) {
     if (valid) {
         OutC* pout = static_cast<OutC*>(a.out) + bz * a.out_batch_stride + (long long)(col / out_div) * a.out_stride +
                      (long long)(col % out_div) * a.out_stride2;
+        if (a.W0 == 0 && es == 1) {
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int n = j + T * q - a.W0;
-            if (n >= 0 && n < a.W) {
-                const float2 x = (a.out_scale != 1.f) ? cscale(v[q], a.out_scale) : v[q];
-                st_cplx<OutC>(pout + n * es, x);
+            for (int q = 0; q < 16; q++)
+                if (j + T * q < a.W) st_cplx<OutC>(pout + j + T * q, v[q]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const int n = j + T * q - a.W0;
+                if (n >= 0 && n < a.W) st_cplx<OutC>(pout + n * es, v[q]);
             }
         }
     }
@@ -506,13 +502,25 @@ c2r_rows_kernel(RowInvArgs a) {
     OutT* oa = static_cast<OutT*>(a.out[gb]) + (long long)ra * a.out_pitch;
     OutT* ob = oa + a.out_pitch;
     const bool has_a = ra < a.n_rows, has_b = ra + 1 < a.n_rows;
-    if (!a.peaks_only) {
+    if (a.scale != 1.f) {
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int n = j + T * q - a.X0;
-            if (n >= 0 && n < a.W) {
-                if (has_a) st_real<OutT>(oa + n, v[q].x * a.scale);
-                if (has_b) st_real<OutT>(ob + n, v[q].y * a.scale);
+        for (int q = 0; q < 16; q++) v[q] = cscale(v[q], a.scale);
+    }
+    if (!a.peaks_only) {
+        const int Wa = has_a ? a.W : 0, Wb = has_b ? a.W : 0;
+        if (a.X0 == 0) {
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const int n = j + T * q;
+                if (n < Wa) st_real<OutT>(oa + n, v[q].x);
+                if (n < Wb) st_real<OutT>(ob + n, v[q].y);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 16; q++) {
+                const int n = j + T * q - a.X0;
+                if (n >= 0 && n < Wa) st_real<OutT>(oa + n, v[q].x);
+                if (n >= 0 && n < Wb) st_real<OutT>(ob + n, v[q].y);
             }
         }
     }
@@ -523,8 +531,8 @@ c2r_rows_kernel(RowInvArgs a) {
         for (int q = 0; q < 16; q++) {
             const int n = j + T * q - a.X0;
             if (n >= 0 && n < a.W) {
-                if (has_a) atomicMax(ma + n, peak_key(v[q].x * a.scale, tmpl));
-                if (has_b) atomicMax(ma + a.W + n, peak_key(v[q].y * a.scale, tmpl));
+                if (has_a) atomicMax(ma + n, peak_key(v[q].x, tmpl));
+                if (has_b) atomicMax(ma + a.W + n, peak_key(v[q].y, tmpl));
             }
         }
     }
@@ -535,11 +543,11 @@ c2r_rows_kernel(RowInvArgs a) {
             const int n = j + T * q - a.X0;
             if (n >= 0 && n < a.W) {
                 if (has_a) {
-                    const unsigned long long k = peak_key(v[q].x * a.scale, (unsigned)(ra * a.W + n));
+                    const unsigned long long k = peak_key(v[q].x, (unsigned)(ra * a.W + n));
                     best = k > best ? k : best;
                 }
                 if (has_b) {
-                    const unsigned long long k = peak_key(v[q].y * a.scale, (unsigned)((ra + 1) * a.W + n));
+                    const unsigned long long k = peak_key(v[q].y, (unsigned)((ra + 1) * a.W + n));
                     best = k > best ? k : best;
                 }
             }

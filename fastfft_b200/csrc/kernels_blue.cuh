@@ -177,8 +177,7 @@ blue_cols_kernel(ColArgs a, BlueArgs b) {
 #pragma unroll
     for (int q = 0; q < 16; q++) {
         const int n = j + T * q;
-        const float2 x = n < L ? ld_cplx<InC>(pin + n) : make_float2(0.f, 0.f);
-        v[q] = (a.in_scale != 1.f) ? cscale(x, a.in_scale) : x;
+        v[q] = n < L ? ld_cplx<InC>(pin + n) : make_float2(0.f, 0.f);
     }
     const int keep = min(N, a.W0 + a.W);
     if constexpr (MODE == COL_FWD) {

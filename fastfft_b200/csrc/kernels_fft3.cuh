@@ -282,15 +282,11 @@ cols3_kernel(ColArgs a) {
 #pragma unroll
         for (int q = 0; q < 16; q++) {
             const int k = R * (j + TP * q) + k2;
-            const float2 x = (valid && k < a.L) ? ld_cplx<InC>(pin + k) : make_float2(0.f, 0.f);
-            v[q] = (a.in_scale != 1.f) ? cscale(x, a.in_scale) : x;
+            v[q] = (valid && k < a.L) ? ld_cplx<InC>(pin + k) : make_float2(0.f, 0.f);
         }
         BlockFft<P, true>::run(v, g, j, a.tw, 16);
     } else {
-        auto ld = [&](int n) {
-            const float2 x = (valid && n < a.L) ? ld_cplx<InC>(pin + n) : make_float2(0.f, 0.f);
-            return (a.in_scale != 1.f) ? cscale(x, a.in_scale) : x;
-        };
+        auto ld = [&](int n) { return (valid && n < a.L) ? ld_cplx<InC>(pin + n) : make_float2(0.f, 0.f); };
 #pragma unroll
         for (int q = 0; q < 16; q++) {
             const int n1 = j + TP * q;

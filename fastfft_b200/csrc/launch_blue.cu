@@ -6,8 +6,7 @@
 #include <mutex>
 #include <utility>
 
-#include "kernels_blue.cuh"
-#include "launch_common.cuh"
+#include "launch_blue.cuh"
 
 namespace ffb {
 
@@ -96,134 +95,18 @@ cudaError_t blue_tables(int n, BlueArgs* b) {
     return cudaSuccess;
 }
 
-template <int M>
-constexpr size_t blue_smem() {
-    return (size_t)FftGroup<M, 1, true>::BYTES;
-}
-
-template <int M, class InT>
-cudaError_t r2c_impl(const RowFwdArgs& a, const BlueArgs& b, cudaStream_t st) {
-    static std::atomic<int> hw[64];
-    auto fn = blue_r2c_rows_kernel<M, InT>;
-    cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
-    if (e != cudaSuccess) return e;
-    const int grid = (a.n_rows + 1) / 2;
-    if (grid == 0) return cudaSuccess;
-    fn<<<dim3(grid, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
-}
-
-template <int M, class OutT>
-cudaError_t c2r_impl(const RowInvArgs& a, const BlueArgs& b, cudaStream_t st) {
-    static std::atomic<int> hw[64];
-    auto fn = blue_c2r_rows_kernel<M, OutT>;
-    cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
-    if (e != cudaSuccess) return e;
-    const int grid = (a.n_rows + 1) / 2;
-    if (grid == 0) return cudaSuccess;
-    fn<<<dim3(grid, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
-}
-
-template <int M, class InC>
-cudaError_t c2c_fwd_impl(const RowFwdArgs& a, const BlueArgs& b, cudaStream_t st) {
-    static std::atomic<int> hw[64];
-    auto fn = blue_c2c_rows_fwd_kernel<M, InC>;
-    cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
-    if (e != cudaSuccess) return e;
-    if (a.n_rows == 0) return cudaSuccess;
-    fn<<<dim3(a.n_rows, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
-}
-
-template <int M, class OutC>
-cudaError_t c2c_inv_impl(const RowInvArgs& a, const BlueArgs& b, cudaStream_t st) {
-    static std::atomic<int> hw[64];
-    auto fn = blue_c2c_rows_inv_kernel<M, OutC>;
-    cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
-    if (e != cudaSuccess) return e;
-    if (a.n_rows == 0) return cudaSuccess;
-    fn<<<dim3(a.n_rows, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
-}
-
-template <int M, int MODE, class InC, class ImgC, class OutC>
-cudaError_t cols_impl(const ColArgs& a, const BlueArgs& b, cudaStream_t st) {
-    static std::atomic<int> hw[64];
-    auto fn = blue_cols_kernel<M, MODE, InC, ImgC, OutC>;
-    cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
-    if (e != cudaSuccess) return e;
-    if (a.n_cols == 0) return cudaSuccess;
-    fn<<<dim3(a.n_cols, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
-}
-
-template <int M>
-cudaError_t r2c_m(int in_dtype, const RowFwdArgs& a, const BlueArgs& b, cudaStream_t st) {
-    switch (in_dtype) {
-        case 0: return r2c_impl<M, float>(a, b, st);
-        case 1: return r2c_impl<M, __half>(a, b, st);
-        case 2: return r2c_impl<M, __nv_bfloat16>(a, b, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-template <int M>
-cudaError_t c2r_m(int out_dtype, const RowInvArgs& a, const BlueArgs& b, cudaStream_t st) {
-    switch (out_dtype) {
-        case 0: return c2r_impl<M, float>(a, b, st);
-        case 1: return c2r_impl<M, __half>(a, b, st);
-        case 2: return c2r_impl<M, __nv_bfloat16>(a, b, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-// complex storage: 3 float2, 4 __half2, 5 __nv_bfloat162
-template <int M>
-cudaError_t c2c_fwd_m(int in_dtype, const RowFwdArgs& a, const BlueArgs& b, cudaStream_t st) {
-    switch (in_dtype) {
-        case 3: return c2c_fwd_impl<M, float2>(a, b, st);
-        case 4: return c2c_fwd_impl<M, __half2>(a, b, st);
-        case 5: return c2c_fwd_impl<M, __nv_bfloat162>(a, b, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-template <int M>
-cudaError_t c2c_inv_m(int out_dtype, const RowInvArgs& a, const BlueArgs& b, cudaStream_t st) {
-    switch (out_dtype) {
-        case 3: return c2c_inv_impl<M, float2>(a, b, st);
-        case 4: return c2c_inv_impl<M, __half2>(a, b, st);
-        case 5: return c2c_inv_impl<M, __nv_bfloat162>(a, b, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-// dtype: the output storage (FWD), the input storage (INV) or the image storage (XCORR), as the
-// power-of-two column launchers take it
-template <int M>
-cudaError_t cols_m(int mode, int dtype, const ColArgs& a, const BlueArgs& b, cudaStream_t st) {
-    if (mode == COL_FWD) {
-        switch (dtype) {
-            case 3: return cols_impl<M, COL_FWD, float2, float2, float2>(a, b, st);
-            case 4: return cols_impl<M, COL_FWD, float2, float2, __half2>(a, b, st);
-            case 5: return cols_impl<M, COL_FWD, float2, float2, __nv_bfloat162>(a, b, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    if (mode == COL_INV) {
-        switch (dtype) {
-            case 3: return cols_impl<M, COL_INV, float2, float2, float2>(a, b, st);
-            case 4: return cols_impl<M, COL_INV, __half2, float2, float2>(a, b, st);
-            case 5: return cols_impl<M, COL_INV, __nv_bfloat162, float2, float2>(a, b, st);
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    switch (dtype) {
-        case 3: return cols_impl<M, COL_XCORR, float2, float2, float2>(a, b, st);
-        case 4: return cols_impl<M, COL_XCORR, float2, __half2, float2>(a, b, st);
-        case 5: return cols_impl<M, COL_XCORR, float2, __nv_bfloat162, float2>(a, b, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-
 }  // namespace
+
+namespace blue {
+FFB_BLUE_LAUNCHERS(, 64)
+FFB_BLUE_LAUNCHERS(, 128)
+FFB_BLUE_LAUNCHERS(, 256)
+FFB_BLUE_LAUNCHERS(, 512)
+FFB_BLUE_LAUNCHERS(extern, 1024)
+FFB_BLUE_LAUNCHERS(extern, 2048)
+FFB_BLUE_LAUNCHERS(extern, 4096)
+FFB_BLUE_LAUNCHERS(extern, 8192)
+}  // namespace blue
 
 cudaError_t prepare_blue_tables(int n) {
     if (!is_blue_size(n)) return cudaErrorInvalidValue;
@@ -233,14 +116,14 @@ cudaError_t prepare_blue_tables(int n) {
 
 #define FFB_BLUE_M_SWITCH(n, FN, ...)                  \
     switch (blue_m(n)) {                               \
-        case 64: return FN<64>(__VA_ARGS__);           \
-        case 128: return FN<128>(__VA_ARGS__);         \
-        case 256: return FN<256>(__VA_ARGS__);         \
-        case 512: return FN<512>(__VA_ARGS__);         \
-        case 1024: return FN<1024>(__VA_ARGS__);       \
-        case 2048: return FN<2048>(__VA_ARGS__);       \
-        case 4096: return FN<4096>(__VA_ARGS__);       \
-        case 8192: return FN<8192>(__VA_ARGS__);       \
+        case 64: return blue::FN<64>(__VA_ARGS__);           \
+        case 128: return blue::FN<128>(__VA_ARGS__);         \
+        case 256: return blue::FN<256>(__VA_ARGS__);         \
+        case 512: return blue::FN<512>(__VA_ARGS__);         \
+        case 1024: return blue::FN<1024>(__VA_ARGS__);       \
+        case 2048: return blue::FN<2048>(__VA_ARGS__);       \
+        case 4096: return blue::FN<4096>(__VA_ARGS__);       \
+        case 8192: return blue::FN<8192>(__VA_ARGS__);       \
         default: return cudaErrorInvalidValue;         \
     }
 

@@ -140,7 +140,6 @@ extern "C" fastfft_status fastfft_fwd_image_inv_2d_noalloc(const float* input, i
     c.n_cols = (int)kx;
     c.intra_kind = intra_op ? intra_op->kind : FASTFFT_OP_NOOP;
     c.intra_scale = intra_op ? intra_op->scale : 1.f;
-    c.in_scale = 1.f;
     c.out_scale = 1.f;
     c.tw = tw;
     c.n_batch = 1;

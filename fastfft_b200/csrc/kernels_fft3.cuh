@@ -57,6 +57,7 @@ r2c3_rows_kernel(RowFwdArgs a) {
     const int n_rows = a.rows_g[gb] > 0 ? a.rows_g[gb] : a.n_rows;
     const int L = a.L_g[gb] > 0 ? a.L_g[gb] : a.L;
     const long long in_pitch = a.pitch_g[gb] > 0 ? a.pitch_g[gb] : a.in_pitch;
+    if (2 * blockIdx.x * FPB >= n_rows) return;   // (block-uniform) an uneven batch's shorter template
     const int ra = 2 * (blockIdx.x * FPB + f);
     const bool has_a = ra < n_rows, has_b = ra + 1 < n_rows;
     const InT* in_g = static_cast<const InT*>(a.in[gb]);

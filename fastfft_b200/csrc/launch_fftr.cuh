@@ -6,6 +6,7 @@
 #pragma once
 
 #include "kernels_fft3.cuh"
+#include "kernels_rows_split.cuh"
 #include "launch_common.cuh"
 
 namespace ffb {
@@ -69,9 +70,56 @@ static cudaError_t tables3(int r, int p, const float2** tw, const float2** tw3) 
     return twiddles_for(r * p, tw3);
 }
 
+// Row passes on the split block FFT, at the lengths where they are the faster form.  Measured on
+// B200 (us per launch, before / split): R2C 1536 (64 templates of 384 rows) 75.5 / 62.9, 384 (12 of
+// 96) 12.0 / 9.6; C2R 1536 (64 windows of 1024 rows) 184 / 167, one window of 777 rows 12.1 / 11.3,
+// 384 (12 of 256) 10.1 / 8.9.  768 keeps the radix-3 form (R2C 22.8 / 24.1 and C2R 24.4 / 25.3 per 32),
+// and powers of two theirs (1024: R2C 25.6 / 26.1, C2R 32.1 / 33.2 per 32).
+constexpr bool split_rows_size(int n) { return n == 1536 || n == 384; }
+template <int N>
+constexpr int split_rows_fpb() {
+    return N == 1536 ? 4 : 8;
+}
+template <int N, class InT>
+static cudaError_t r2c_split_impl(const RowFwdArgs& a0, cudaStream_t st) {
+    constexpr int FPB = split_rows_fpb<N>(), MINB = N == 1536 ? 3 : 4;
+    using SR = SplitRows<N, FPB>;
+    RowFwdArgs a = a0;
+    cudaError_t e = split_twiddles_for(N, &a.tw);
+    if (e != cudaSuccess) return e;
+    static std::atomic<unsigned long long> mask{0};
+    auto fn = r2c_split_rows_kernel<N, InT, FPB, MINB>;
+    if ((e = ensure_smem_attr((const void*)fn, SR::BYTES, &mask)) != cudaSuccess) return e;
+    const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
+    if (grid == 0) return cudaSuccess;
+    if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
+    fn<<<dim3(grid, a.n_batch), SR::T * FPB, SR::BYTES, st>>>(a);
+    return cudaGetLastError();
+}
+template <int N, class OutT>
+static cudaError_t c2r_split_impl(const RowInvArgs& a0, cudaStream_t st) {
+        constexpr int FPB = split_rows_fpb<N>(), MINB = N == 1536 ? 3 : 4;
+    using SR = SplitRows<N, FPB>;
+    RowInvArgs a = a0;
+    cudaError_t e = split_twiddles_for(N, &a.tw);
+    if (e != cudaSuccess) return e;
+    static std::atomic<unsigned long long> mask_plain{0}, mask_full{0};
+    const bool plain = !a.peaks && !a.mip && !a.peaks_only && a.X0 == 0;
+    auto fn = plain ? c2r_split_rows_kernel<N, OutT, FPB, MINB, true> : c2r_split_rows_kernel<N, OutT, FPB, MINB, false>;
+    if ((e = ensure_smem_attr((const void*)fn, SR::BYTES, plain ? &mask_plain : &mask_full)) != cudaSuccess) return e;
+    const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
+    if (grid == 0) return cudaSuccess;
+    if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
+    fn<<<dim3(grid, a.n_batch), SR::T * FPB, SR::BYTES, st>>>(a);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 template <int R, int P, class InT>
 static cudaError_t r2c3_impl(const RowFwdArgs& a0, cudaStream_t st) {
+    if constexpr (split_rows_size(R * P)) {
+        return r2c_split_impl<R * P, InT>(a0, st);
+    } else {
     constexpr int FPB = row_fpb3<R, P>();
     constexpr int THREADS = FftRShape<R, P>::T * FPB;
     const size_t smem = (size_t)FftRGroup<R, P, FPB, false>::BYTES;
@@ -86,6 +134,7 @@ static cudaError_t r2c3_impl(const RowFwdArgs& a0, cudaStream_t st) {
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
     fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
     return cudaGetLastError();
+    }
 }
 
 template <int R, int P>
@@ -106,6 +155,9 @@ cudaError_t launch_r2c_r(int n, int in_dtype, const RowFwdArgs& a, cudaStream_t 
 // ---------------------------------------------------------------------------
 template <int R, int P, class OutT>
 static cudaError_t c2r3_impl(const RowInvArgs& a0, cudaStream_t st) {
+    if constexpr (split_rows_size(R * P)) {
+        return c2r_split_impl<R * P, OutT>(a0, st);
+    } else {
     constexpr int FPB = row_fpb3<R, P>();
     constexpr int THREADS = FftRShape<R, P>::T * FPB;
     const size_t smem = (size_t)FftRGroup<R, P, FPB, false, FftRShape<R, P>::SUB_C2R, FftRShape<R, P>::C2R_FFT_EXTRA>::BYTES;
@@ -122,6 +174,7 @@ static cudaError_t c2r3_impl(const RowInvArgs& a0, cudaStream_t st) {
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
     fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
     return cudaGetLastError();
+    }
 }
 
 template <int R, int P>

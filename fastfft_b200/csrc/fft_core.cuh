@@ -21,6 +21,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "grid_dep.cuh"
+
 #ifndef FFB_PACKED_F32X2
 #define FFB_PACKED_F32X2 0
 #endif

@@ -25,11 +25,12 @@ namespace ffb {
 // ---------------------------------------------------------------------------
 // dtype helpers
 // ---------------------------------------------------------------------------
+// (plain loads: one through the read-only path may be moved above grid_dependency())
 template <class T> __device__ __forceinline__ float ld_real(const T* p);
-template <> __device__ __forceinline__ float ld_real<float>(const float* p) { return __ldg(p); }
-template <> __device__ __forceinline__ float ld_real<__half>(const __half* p) { return __half2float(__ldg(p)); }
+template <> __device__ __forceinline__ float ld_real<float>(const float* p) { return *p; }
+template <> __device__ __forceinline__ float ld_real<__half>(const __half* p) { return __half2float(*p); }
 template <> __device__ __forceinline__ float ld_real<__nv_bfloat16>(const __nv_bfloat16* p) {
-    return __bfloat162float(__ldg(p));
+    return __bfloat162float(*p);
 }
 
 template <class T> __device__ __forceinline__ void st_real(T* p, float v);
@@ -139,6 +140,7 @@ __device__ __forceinline__ long long input_row(int r, int rows_y, int rows_z) {
 template <int N, class InT, int FPB>
 __global__ void __launch_bounds__(FftShape<N>::T * FPB, (FftShape<N>::T * FPB <= 256) ? 4 : 2)
 r2c_rows_kernel(RowFwdArgs a) {
+    grid_dependency();
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ float2 smem[];
@@ -279,6 +281,7 @@ struct ColSmem {
 template <int N, int MODE, class InC, class ImgC, class OutC, int FPB>
 __global__ void __launch_bounds__(FftShape<N>::T * FPB, ColGroup<N, MODE, FPB>::kMinBlocks)
 cols_kernel(ColArgs a) {
+    grid_dependency();
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ __align__(128) float2 smem[];
@@ -438,6 +441,7 @@ __device__ __forceinline__ unsigned long long peak_key(float v, unsigned int ind
 template <int N, class OutT, int FPB>
 __global__ void __launch_bounds__(FftShape<N>::T * FPB, (FftShape<N>::T * FPB <= 256) ? 4 : 2)
 c2r_rows_kernel(RowInvArgs a) {
+    grid_dependency();
     using S = FftShape<N>;
     constexpr int T = S::T;
     constexpr int H = N / 2;

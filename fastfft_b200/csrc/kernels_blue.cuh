@@ -55,6 +55,7 @@ __device__ __forceinline__ void bluestein_dft(float2 (&v)[16], G& g, int j, cons
 template <int M, class InT>
 __global__ void __launch_bounds__(M / 16)
 blue_r2c_rows_kernel(RowFwdArgs a, BlueArgs b) {
+    grid_dependency();
     constexpr int T = M / 16;
     extern __shared__ float2 smem[];
     using G = FftGroup<M, 1, true>;
@@ -106,6 +107,7 @@ blue_r2c_rows_kernel(RowFwdArgs a, BlueArgs b) {
 template <int M, class OutT>
 __global__ void __launch_bounds__(M / 16)
 blue_c2r_rows_kernel(RowInvArgs a, BlueArgs b) {
+    grid_dependency();
     constexpr int T = M / 16;
     extern __shared__ float2 smem[];
     using G = FftGroup<M, 1, true>;
@@ -161,6 +163,7 @@ blue_c2r_rows_kernel(RowInvArgs a, BlueArgs b) {
 template <int M, int MODE, class InC, class ImgC, class OutC>
 __global__ void __launch_bounds__(M / 16)
 blue_cols_kernel(ColArgs a, BlueArgs b) {
+    grid_dependency();
     constexpr int T = M / 16;
     extern __shared__ float2 smem[];
     using G = FftGroup<M, 1, true>;
@@ -218,6 +221,7 @@ blue_cols_kernel(ColArgs a, BlueArgs b) {
 template <int M, class InC>
 __global__ void __launch_bounds__(M / 16)
 blue_c2c_rows_fwd_kernel(RowFwdArgs a, BlueArgs b) {
+    grid_dependency();
     constexpr int T = M / 16;
     extern __shared__ float2 smem[];
     using G = FftGroup<M, 1, true>;
@@ -249,6 +253,7 @@ blue_c2c_rows_fwd_kernel(RowFwdArgs a, BlueArgs b) {
 template <int M, class OutC>
 __global__ void __launch_bounds__(M / 16)
 blue_c2c_rows_inv_kernel(RowInvArgs a, BlueArgs b) {
+    grid_dependency();
     constexpr int T = M / 16;
     extern __shared__ float2 smem[];
     using G = FftGroup<M, 1, true>;

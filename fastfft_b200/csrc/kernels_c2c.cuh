@@ -22,6 +22,7 @@ namespace ffb {
 template <int N, class InC, int FPB>
 __global__ void __launch_bounds__(FftShape<N>::T * FPB, (FftShape<N>::T * FPB <= 256) ? 4 : 2)
 c2c_rows_fwd_kernel(RowFwdArgs a) {
+    grid_dependency();
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ float2 smem[];
@@ -58,6 +59,7 @@ c2c_rows_fwd_kernel(RowFwdArgs a) {
 template <int N, class OutC, int FPB>
 __global__ void __launch_bounds__(FftShape<N>::T * FPB, (FftShape<N>::T * FPB <= 256) ? 4 : 2)
 c2c_rows_inv_kernel(RowInvArgs a) {
+    grid_dependency();
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ float2 smem[];

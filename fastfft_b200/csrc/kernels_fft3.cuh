@@ -39,6 +39,7 @@ constexpr int kXcorr3SmThreads = FFB_XCORR3_SM_THREADS;
 template <int R, int P, class InT, int FPB>
 __global__ void __launch_bounds__(FftRShape<R, P>::T * FPB, FFB_ROWS3_MIN_BLOCKS)
 r2c3_rows_kernel(RowFwdArgs a) {
+    grid_dependency();
     using S3 = FftRShape<R, P>;
     constexpr int N = S3::N;
     constexpr int T = S3::T;
@@ -125,6 +126,7 @@ r2c3_rows_kernel(RowFwdArgs a) {
 template <int R, int P, class OutT, int FPB, bool PLAIN>
 __global__ void __launch_bounds__(FftRShape<R, P>::T * FPB, FFB_C2R3_MIN_BLOCKS)
 c2r3_rows_kernel(RowInvArgs a) {
+    grid_dependency();
     using S3 = FftRShape<R, P>;
     constexpr int N = S3::N;
     constexpr int T = S3::T;
@@ -262,6 +264,7 @@ template <int R, int P, int MODE, class InC, class ImgC, int FPB, class OutC = f
 __global__ void __launch_bounds__(FftRShape<R, P>::T * FPB, FftRShape<R, P>::T * FPB < kXcorr3SmThreads
                                                                 ? kXcorr3SmThreads / (FftRShape<R, P>::T * FPB) : 1)
 cols3_kernel(ColArgs a) {
+    grid_dependency();
     using S3 = FftRShape<R, P>;
     constexpr int T = S3::T;
     constexpr int TP = S3::TP;
@@ -360,6 +363,7 @@ template <int R, int P, class ImgC, int FPB>
 __global__ void __launch_bounds__(FftRShape<R, P>::T * FPB,
                                   FftRShape<R, P>::T * FPB < kXcorr3SmThreads ? kXcorr3SmThreads / (FftRShape<R, P>::T * FPB) : 1)
 xcorr3_cols_kernel(XcorrColArgs a) {
+    grid_dependency();
     using S3 = FftRShape<R, P>;
     using SM = Xcorr3Smem<R, P, ImgC, FPB>;
     constexpr int T = S3::T;

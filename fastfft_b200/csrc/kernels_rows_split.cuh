@@ -50,6 +50,7 @@ __device__ __forceinline__ void split_sync(int f) {
 template <int N, class InT, int FPB, int MIN_BLOCKS>
 __global__ void __launch_bounds__(SplitRows<N, FPB>::T * FPB, MIN_BLOCKS)
 r2c_split_rows_kernel(RowFwdArgs a) {
+    grid_dependency();
     using SR = SplitRows<N, FPB>;
     using F = typename SR::F;
     constexpr int T = SR::T, E = SR::E;
@@ -115,6 +116,7 @@ r2c_split_rows_kernel(RowFwdArgs a) {
 template <int N, class OutT, int FPB, int MIN_BLOCKS, bool PLAIN>
 __global__ void __launch_bounds__(SplitRows<N, FPB>::T * FPB, MIN_BLOCKS)
 c2r_split_rows_kernel(RowInvArgs a) {
+    grid_dependency();
     using SR = SplitRows<N, FPB>;
     using F = typename SR::F;
     constexpr int T = SR::T, E = SR::E, H = N / 2;

@@ -79,6 +79,7 @@ template <int N, class ImgC, int FPB>
 __global__ void __launch_bounds__(FftShape<N>::T * FPB,
                                   FftShape<N>::T * FPB < kXcorrSmThreads ? kXcorrSmThreads / (FftShape<N>::T * FPB) : 1)
 xcorr_cols_kernel(XcorrColArgs a) {
+    grid_dependency();
     using S = FftShape<N>;
     using SM = XcorrSmem<N, ImgC, FPB>;
     constexpr int T = S::T;
@@ -195,6 +196,7 @@ struct XcorrSplitSmem {
 template <int N, class C, int G, int MIN_BLOCKS>
 __global__ void __launch_bounds__(SplitFft<N, C>::T * G, MIN_BLOCKS)
 xcorr_split_kernel(XcorrColArgs a) {
+    grid_dependency();
     using F = SplitFft<N, C>;
     using SM = XcorrSplitSmem<N, C, G>;
     constexpr int T = F::T, E = F::E, W = SM::W;

@@ -22,8 +22,7 @@ cudaError_t r2c_impl(const RowFwdArgs& a, const BlueArgs& b, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const int grid = (a.n_rows + 1) / 2;
     if (grid == 0) return cudaSuccess;
-    fn<<<dim3(grid, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), M / 16, blue_smem<M>(), st, a, b);
 }
 
 template <int M, class OutT>
@@ -34,8 +33,7 @@ cudaError_t c2r_impl(const RowInvArgs& a, const BlueArgs& b, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const int grid = (a.n_rows + 1) / 2;
     if (grid == 0) return cudaSuccess;
-    fn<<<dim3(grid, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), M / 16, blue_smem<M>(), st, a, b);
 }
 
 template <int M, class InC>
@@ -45,8 +43,7 @@ cudaError_t c2c_fwd_impl(const RowFwdArgs& a, const BlueArgs& b, cudaStream_t st
     cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
     if (e != cudaSuccess) return e;
     if (a.n_rows == 0) return cudaSuccess;
-    fn<<<dim3(a.n_rows, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(a.n_rows, a.n_batch), M / 16, blue_smem<M>(), st, a, b);
 }
 
 template <int M, class OutC>
@@ -56,8 +53,7 @@ cudaError_t c2c_inv_impl(const RowInvArgs& a, const BlueArgs& b, cudaStream_t st
     cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
     if (e != cudaSuccess) return e;
     if (a.n_rows == 0) return cudaSuccess;
-    fn<<<dim3(a.n_rows, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(a.n_rows, a.n_batch), M / 16, blue_smem<M>(), st, a, b);
 }
 
 template <int M, int MODE, class InC, class ImgC, class OutC>
@@ -67,8 +63,7 @@ cudaError_t cols_impl(const ColArgs& a, const BlueArgs& b, cudaStream_t st) {
     cudaError_t e = ensure_smem_at_least((const void*)fn, blue_smem<M>(), hw);
     if (e != cudaSuccess) return e;
     if (a.n_cols == 0) return cudaSuccess;
-    fn<<<dim3(a.n_cols, a.n_batch), M / 16, blue_smem<M>(), st>>>(a, b);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(a.n_cols, a.n_batch), M / 16, blue_smem<M>(), st, a, b);
 }
 
 template <int M>

@@ -30,8 +30,7 @@ static cudaError_t cols_impl(const ColArgs& args, cudaStream_t st) {
     const int grid = (a.n_cols + FPB - 1) / FPB;
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
 }
 
 template <int N>

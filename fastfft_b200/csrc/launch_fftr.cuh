@@ -93,8 +93,7 @@ static cudaError_t r2c_split_impl(const RowFwdArgs& a0, cudaStream_t st) {
     const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), SR::T * FPB, SR::BYTES, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), SR::T * FPB, SR::BYTES, st, a);
 }
 template <int N, class OutT>
 static cudaError_t c2r_split_impl(const RowInvArgs& a0, cudaStream_t st) {
@@ -110,8 +109,7 @@ static cudaError_t c2r_split_impl(const RowInvArgs& a0, cudaStream_t st) {
     const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), SR::T * FPB, SR::BYTES, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), SR::T * FPB, SR::BYTES, st, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -132,8 +130,7 @@ static cudaError_t r2c3_impl(const RowFwdArgs& a0, cudaStream_t st) {
     const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
     }
 }
 
@@ -172,8 +169,7 @@ static cudaError_t c2r3_impl(const RowInvArgs& a0, cudaStream_t st) {
     const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
     }
 }
 
@@ -209,8 +205,7 @@ static cudaError_t cols3_impl(const ColArgs& a0, cudaStream_t st) {
     const int grid = (a.n_cols + FPB - 1) / FPB;
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
 }
 
 template <int R, int P>
@@ -275,8 +270,7 @@ static cudaError_t xcorr3_impl(const XcorrColArgs& a0, cudaStream_t st) {
     static std::atomic<int> high_water[64];
     auto fn = xcorr3_cols_kernel<R, P, ImgC, FPB>;
     if ((e = ensure_smem_at_least((const void*)fn, (size_t)smem, high_water)) != cudaSuccess) return e;
-    fn<<<dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), FftRShape<R, P>::T * FPB, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), FftRShape<R, P>::T * FPB, smem, st, a);
     }
 }
 

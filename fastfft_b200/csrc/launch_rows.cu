@@ -16,8 +16,7 @@ static cudaError_t r2c_impl(const RowFwdArgs& a, cudaStream_t st) {
     const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
 }
 
 template <int N>
@@ -48,8 +47,7 @@ static cudaError_t c2r_impl(const RowInvArgs& a, cudaStream_t st) {
     const int grid = (a.n_rows + 2 * FPB - 1) / (2 * FPB);
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
 }
 
 template <int N>
@@ -81,8 +79,7 @@ static cudaError_t c2c_fwd_impl(const RowFwdArgs& a, cudaStream_t st) {
     const int grid = (a.n_rows + FPB - 1) / FPB;
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch || a.kmax > N) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
 }
 
 template <int N>
@@ -112,8 +109,7 @@ static cudaError_t c2c_inv_impl(const RowInvArgs& a, cudaStream_t st) {
     const int grid = (a.n_rows + FPB - 1) / FPB;
     if (grid == 0) return cudaSuccess;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch) return cudaErrorInvalidValue;
-    fn<<<dim3(grid, a.n_batch), THREADS, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(grid, a.n_batch), THREADS, smem, st, a);
 }
 
 template <int N>

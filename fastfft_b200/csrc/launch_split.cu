@@ -12,8 +12,7 @@ static cudaError_t xcorr_split_impl(const XcorrColArgs& a, cudaStream_t st) {
     auto fn = xcorr_split_kernel<N, C, G, MIN_BLOCKS>;
     cudaError_t e = ensure_smem_at_least((const void*)fn, (size_t)smem, high_water);
     if (e != cudaSuccess) return e;
-    fn<<<dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), SplitFft<N, C>::T * G, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(fn, dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), SplitFft<N, C>::T * G, smem, st, a);
 }
 
 // Blocks of G transform groups; registers for MIN_BLOCKS blocks per SM.  Measured on B200 (us per

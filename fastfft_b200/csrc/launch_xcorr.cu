@@ -29,8 +29,7 @@ static cudaError_t xcorr_v2_impl(const XcorrColArgs& a, cudaStream_t st) {
         auto fn = xcorr_cols_kernel<N, ImgC, FPB>;
         cudaError_t e = ensure_smem_at_least((const void*)fn, (size_t)smem, high_water);
         if (e != cudaSuccess) return e;
-        fn<<<dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), FftShape<N>::T * FPB, smem, st>>>(a);
-        return cudaGetLastError();
+        return launch_dependent(fn, dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), FftShape<N>::T * FPB, smem, st, a);
     }
 }
 

@@ -51,16 +51,40 @@ class KernelFunction:
         return C.fastfft_op(C.OP_CONJ_MUL_THEN_SCALE, float(s))
 
 
+_torch = None   # the torch module, once a plan has been bound to one of its streams
+
+
 def _ptr(x) -> int | None:
-    if x is None:
-        return None
-    if isinstance(x, int):
+    if x is None or isinstance(x, int):
         return x
-    if hasattr(x, "data_ptr"):
-        if hasattr(x, "is_cuda") and not x.is_cuda:
-            raise ValueError("FastFFT buffers must be CUDA device memory")
-        return x.data_ptr()
-    raise TypeError(f"cannot take a device pointer of {type(x)}")
+    try:
+        data_ptr = x.data_ptr
+    except AttributeError:
+        raise TypeError(f"cannot take a device pointer of {type(x)}") from None
+    if not getattr(x, "is_cuda", True):
+        raise ValueError("FastFFT buffers must be CUDA device memory")
+    return data_ptr()
+
+
+def _ptr_array(xs):
+    """A C array of the device pointers of a list of buffers."""
+    return (ctypes.c_void_p * len(xs))(*[_ptr(x) for x in xs])
+
+
+def _fits(xs, n):
+    """Whether an optional list holds one entry per template."""
+    return xs is None or len(xs) == n
+
+
+def _images_fit(images, n):
+    return not isinstance(images, (list, tuple)) or len(images) == n
+
+
+def _image_array(images, n):
+    """The image pointer of each of n templates: one image for all of them, or a list."""
+    if not isinstance(images, (list, tuple)):
+        return (ctypes.c_void_p * n)(*([_ptr(images)] * n if n else []))
+    return _ptr_array(images)
 
 
 def _opref(op):
@@ -88,6 +112,7 @@ class FourierTransformer:
         if st != C.OK:
             raise C.FastFFTError(st, self._lib.fastfft_last_error(None).decode())
         self._stream = None
+        self._raw_stream = None   # the torch stream the plan was last bound to
         self.rank = rank
         self.complex_input = str(input_dtype).replace("torch.", "") in _CPLX_DTYPES
 
@@ -107,14 +132,25 @@ class FourierTransformer:
             raise C.FastFFTError(st, self._lib.fastfft_last_error(self._h).decode())
 
     def _bind_stream(self):
+        global _torch
         if self._stream is not None:
             return
-        try:
-            import torch
-        except ImportError:  # pragma: no cover - torch is part of the image
-            return
-        if torch.cuda.is_available():
-            self._check(self._lib.fastfft_set_stream(self._h, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        if self._raw_stream is not None:
+            # torch and its CUDA state are up: the raw handle of the current stream, which the
+            # plan is told only when it changes (about 5 us of a 13 us call otherwise)
+            raw = _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
+            if raw == self._raw_stream:
+                return
+        else:
+            try:
+                import torch as _torch
+            except ImportError:  # pragma: no cover - torch is part of the image
+                return
+            if not _torch.cuda.is_available():
+                return
+            raw = _torch.cuda.current_stream().cuda_stream
+        self._check(self._lib.fastfft_set_stream(self._h, raw))
+        self._raw_stream = raw
 
     # -- plans -----------------------------------------------------------
     def SetForwardFFTPlan(self, ix, iy, iz, ox, oy, oz, is_padded_output=True):
@@ -161,16 +197,13 @@ class FourierTransformer:
         template; outputs is a list of the same length as inputs, or None (in place).
         """
         n = len(inputs)
-        if not isinstance(images, (list, tuple)):
-            images = [images] * n
-        if len(images) != n or (outputs is not None and len(outputs) != n):
+        if not (_images_fit(images, n) and _fits(outputs, n)):
             raise ValueError("inputs, images and outputs must have the same length")
         if intra_op is None:
             intra_op = KernelFunction.conj_mul()
-        arr = ctypes.c_void_p * n
-        ins = arr(*[_ptr(x) for x in inputs])
-        ims = arr(*[_ptr(x) for x in images])
-        outs = arr(*[_ptr(x) for x in outputs]) if outputs is not None else None
+        ins = _ptr_array(inputs)
+        ims = _image_array(images, n)
+        outs = _ptr_array(outputs) if outputs is not None else None
         self._bind_stream()
         self._check(self._lib.fastfft_fwd_image_inv_many(self._h, n, ins, ims, outs, _opref(pre_op), _opref(intra_op),
                                                          _opref(post_op)))
@@ -179,17 +212,14 @@ class FourierTransformer:
                                 post_op=None):
         """FwdImageInvFFTMany for templates of uneven sizes: sizes[i] = (x, y) of template i."""
         n = len(inputs)
-        if not isinstance(images, (list, tuple)):
-            images = [images] * n
-        if len(sizes) != n or len(images) != n or (outputs is not None and len(outputs) != n):
+        if len(sizes) != n or not (_images_fit(images, n) and _fits(outputs, n)):
             raise ValueError("inputs, sizes, images and outputs must have the same length")
         if intra_op is None:
             intra_op = KernelFunction.conj_mul()
-        arr = ctypes.c_void_p * n
         dims = (ctypes.c_int * (2 * n))(*[int(v) for xy in sizes for v in xy])
-        ins = arr(*[_ptr(x) for x in inputs])
-        ims = arr(*[_ptr(x) for x in images])
-        outs = arr(*[_ptr(x) for x in outputs]) if outputs is not None else None
+        ins = _ptr_array(inputs)
+        ims = _image_array(images, n)
+        outs = _ptr_array(outputs) if outputs is not None else None
         self._bind_stream()
         self._check(self._lib.fastfft_fwd_image_inv_many_sized(self._h, n, ins, dims, ims, outs, _opref(pre_op),
                                                                _opref(intra_op), _opref(post_op)))
@@ -199,19 +229,16 @@ class FourierTransformer:
         """Batched correlation with a fused peak search into `peaks` (int64 CUDA tensor, one per
         template; decode with decode_peaks).  outputs None: the windows are not written."""
         n = len(inputs)
-        if not isinstance(images, (list, tuple)):
-            images = [images] * n
-        if len(images) != n or (outputs is not None and len(outputs) != n) or (sizes is not None and len(sizes) != n):
+        if not (_images_fit(images, n) and _fits(outputs, n) and _fits(sizes, n)):
             raise ValueError("inputs, images, sizes and outputs must have the same length")
         if peaks.numel() < n or peaks.element_size() != 8:
             raise ValueError("peaks must hold one 64-bit value per template")
         if intra_op is None:
             intra_op = KernelFunction.conj_mul()
-        arr = ctypes.c_void_p * n
         dims = (ctypes.c_int * (2 * n))(*[int(v) for xy in sizes for v in xy]) if sizes is not None else None
-        ins = arr(*[_ptr(x) for x in inputs])
-        ims = arr(*[_ptr(x) for x in images])
-        outs = arr(*[_ptr(x) for x in outputs]) if outputs is not None else None
+        ins = _ptr_array(inputs)
+        ims = _image_array(images, n)
+        outs = _ptr_array(outputs) if outputs is not None else None
         self._bind_stream()
         self._check(self._lib.fastfft_fwd_image_inv_many_peaks(self._h, n, ins, dims, ims, outs, _ptr(peaks),
                                                                _opref(pre_op), _opref(intra_op), _opref(post_op)))
@@ -224,20 +251,17 @@ class FourierTransformer:
         number index_base + i (decode with decode_peaks).  The array accumulates across
         calls.  outputs None: the windows are not written."""
         n = len(inputs)
-        if not isinstance(images, (list, tuple)):
-            images = [images] * n
-        if len(images) != n or (outputs is not None and len(outputs) != n) or (sizes is not None and len(sizes) != n):
+        if not (_images_fit(images, n) and _fits(outputs, n) and _fits(sizes, n)):
             raise ValueError("inputs, images, sizes and outputs must have the same length")
         out_x, out_y = self.ReturnInvOutputDimensions()[:2]
         if mip.numel() < out_x * out_y or mip.element_size() != 8:
             raise ValueError("mip must hold one 64-bit value per window pixel (out_x * out_y)")
         if intra_op is None:
             intra_op = KernelFunction.conj_mul()
-        arr = ctypes.c_void_p * n
         dims = (ctypes.c_int * (2 * n))(*[int(v) for xy in sizes for v in xy]) if sizes is not None else None
-        ins = arr(*[_ptr(x) for x in inputs])
-        ims = arr(*[_ptr(x) for x in images])
-        outs = arr(*[_ptr(x) for x in outputs]) if outputs is not None else None
+        ins = _ptr_array(inputs)
+        ims = _image_array(images, n)
+        outs = _ptr_array(outputs) if outputs is not None else None
         self._bind_stream()
         self._check(self._lib.fastfft_fwd_image_inv_many_mip(self._h, n, ins, dims, ims, outs, _ptr(mip),
                                                              int(index_base), _opref(pre_op), _opref(intra_op),

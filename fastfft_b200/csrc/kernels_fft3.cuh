@@ -289,6 +289,25 @@ cols3_kernel(ColArgs a) {
             v[q] = (valid && k < a.L) ? ld_cplx<InC>(pin + k) : make_float2(0.f, 0.f);
         }
         BlockFft<P, true>::run(v, g, j, a.tw, 16);
+    } else if constexpr (MODE == COL_FWD) {
+        // decimation in time (as the row R2C): thread (k2, j) loads x[R (j + T' q) + k2], so the
+        // column is read once; in the decimation-in-frequency form below every sub-FFT forms its own
+        // input from all of it (5 * 256 points, 385 columns: 18.1 us that way, 8.8 for the inverse)
+        const int Lc = valid ? a.L : 0;
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            const int n = R * (j + TP * q) + k2;
+            v[q] = n < Lc ? ld_cplx<InC>(pin + n) : make_float2(0.f, 0.f);
+        }
+        const float2* const s = forward_dit<R, P>(v, g, j, t, a.tw, a.tw3, leading_slots_dit<R, P>(Lc, k2, j));
+        if (valid) {
+            OutC* po = static_cast<OutC*>(a.out) + bz * a.out_batch_stride + (long long)col * a.out_stride;
+            for (int n = t; n < a.W; n += T) {
+                const float2 x = s[locR<R, P>(n + a.W0)];
+                st_cplx<OutC>(po + n, (a.out_scale != 1.f) ? cscale(x, a.out_scale) : x);
+            }
+        }
+        return;
     } else {
         auto ld = [&](int n) { return (valid && n < a.L) ? ld_cplx<InC>(pin + n) : make_float2(0.f, 0.f); };
 #pragma unroll
@@ -300,32 +319,19 @@ cols3_kernel(ColArgs a) {
             v[q] = dif_input<R, P>(x, n1, k2, a.tw3);
         }
         BlockFft<P, false>::run(v, g, j, a.tw, valid ? leading_slots_p<P>(a.L, j) : 0);
-        if constexpr (MODE == COL_FWD) {
-            // spectrum side: X[3 m + k2] straight from the registers
-            if (valid) {
-                OutC* po = static_cast<OutC*>(a.out) + bz * a.out_batch_stride + (long long)col * a.out_stride;
+        if (a.intra_kind != 0) {
+            const ImgC* pimg =
+                static_cast<const ImgC*>(a.img) + bz * a.img_batch_stride + (long long)col * a.img_stride;
+            const float sc = a.intra_kind == 3 ? a.intra_scale : 1.f;
 #pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const int n = R * (j + TP * q) + k2 - a.W0;
-                    if (n >= 0 && n < a.W) st_cplx<OutC>(po + n, (a.out_scale != 1.f) ? cscale(v[q], a.out_scale) : v[q]);
-                }
+            for (int q = 0; q < 16; q++) {
+                float2 im = make_float2(0.f, 0.f);
+                if (valid) im = ld_cplx_stream<ImgC>(pimg + R * (j + TP * q) + k2);
+                const float2 pr = conj_mul(v[q], im);
+                v[q] = (sc != 1.f) ? cscale(pr, sc) : pr;
             }
-            return;
-        } else {
-            if (a.intra_kind != 0) {
-                const ImgC* pimg =
-                    static_cast<const ImgC*>(a.img) + bz * a.img_batch_stride + (long long)col * a.img_stride;
-                const float sc = a.intra_kind == 3 ? a.intra_scale : 1.f;
-#pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    float2 im = make_float2(0.f, 0.f);
-                    if (valid) im = ld_cplx_stream<ImgC>(pimg + R * (j + TP * q) + k2);
-                    const float2 pr = conj_mul(v[q], im);
-                    v[q] = (sc != 1.f) ? cscale(pr, sc) : pr;
-                }
-            }
-            BlockFft<P, true>::run(v, g, j, a.tw, 16);
         }
+        BlockFft<P, true>::run(v, g, j, a.tw, 16);
     }
     // INV and XCORR: radix-3 output pass, natural order
     const int W = valid ? a.W : 0;

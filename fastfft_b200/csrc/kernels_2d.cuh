@@ -99,6 +99,15 @@ __device__ __forceinline__ int leading_slots(int L, int j) {
     return q > 16 ? 16 : q;
 }
 
+// float2 per exchange buffer of a block of FPB transforms whose buffers are also walked across the
+// transforms (the row passes' split and gather, the coalesced store of the column passes): at
+// 16 / FPB modulo 16, the FPB x (16 / FPB) elements of a half-warp fall into different banks.
+template <int N, int FPB>
+constexpr int kBlockPad = (FftShape<N>::SMEM + 15) / 16 * 16 + (FPB >= 16 ? 1 : FPB > 1 ? 16 / FPB : 4);
+// Exchange groups of the row passes.
+template <int N, int FPB>
+using RowGroup = FftGroup<N, FPB, false, kBlockPad<N, FPB>>;
+
 // ---------------------------------------------------------------------------
 // Row R2C (forward), two rows per complex FFT
 // ---------------------------------------------------------------------------
@@ -144,7 +153,7 @@ r2c_rows_kernel(RowFwdArgs a) {
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ float2 smem[];
-    using G = FftGroup<N, FPB, false>;
+    using G = RowGroup<N, FPB>;
     const int f = threadIdx.x / T;
     const int j = threadIdx.x - f * T;
     G g(smem, f);
@@ -256,18 +265,16 @@ struct ColArgs {
 // inverse modes keep one buffer per column and registers for four 256-thread blocks per SM: these
 // passes wait for memory, and 32 warps per SM cover that better than the 16 that double
 // buffering and 128 registers left (the correlation, with two transforms per column, keeps
-// those).  The stride of the buffers puts the columns that a half-warp of the coalesced store
-// reads (FPB of them at each element) into different banks; at 4 modulo 16 the 256-point passes
-// read four columns per bank.  The 4096-point passes (one column per block) likewise run better
+// those).  At a buffer stride of 4 modulo 16
+// the 256-point passes also read four columns per bank in the coalesced store.  The 4096-point passes (one column per block) likewise run better
 // with one buffer and four blocks, three for the correlation (24 - 32 instead of 16 - 24 warps per
 // SM; a forward transform of 4096^2 68.0 instead of 71.7 us, a single correlation 54.9 instead of
 // 56.4).
 template <int N, int MODE, int FPB>
 struct ColGroup {
     static constexpr bool kMany = (FPB > 1 && MODE != COL_XCORR) || N == 4096;
-    static constexpr int kPad = (FftShape<N>::SMEM + 15) / 16 * 16 + (FPB >= 16 ? 1 : FPB > 1 ? 16 / FPB : 4);
     static constexpr int kMinBlocks = FftShape<N>::T * FPB > 256 ? 1 : kMany ? (MODE == COL_XCORR ? 3 : 4) : 2;
-    using G = FftGroup<N, FPB, !kMany, kPad>;
+    using G = FftGroup<N, FPB, !kMany, kBlockPad<N, FPB>>;
 };
 
 // Shared-memory plan of cols_kernel (bytes): the FFT groups' exchange buffers, then (when the
@@ -449,7 +456,7 @@ c2r_rows_kernel(RowInvArgs a) {
     constexpr int T = S::T;
     constexpr int H = N / 2;
     extern __shared__ float2 smem[];
-    using G = FftGroup<N, FPB, false>;
+    using G = RowGroup<N, FPB>;
     const int f = threadIdx.x / T;
     const int j = threadIdx.x - f * T;
     G g(smem, f);

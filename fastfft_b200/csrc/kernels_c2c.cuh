@@ -26,7 +26,7 @@ c2c_rows_fwd_kernel(RowFwdArgs a) {
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ float2 smem[];
-    using G = FftGroup<N, FPB, false>;
+    using G = RowGroup<N, FPB>;
     const int f = threadIdx.x / T;
     const int j = threadIdx.x - f * T;
     G g(smem, f);
@@ -63,7 +63,7 @@ c2c_rows_inv_kernel(RowInvArgs a) {
     using S = FftShape<N>;
     constexpr int T = S::T;
     extern __shared__ float2 smem[];
-    using G = FftGroup<N, FPB, false>;
+    using G = RowGroup<N, FPB>;
     const int f = threadIdx.x / T;
     const int j = threadIdx.x - f * T;
     G g(smem, f);

@@ -32,6 +32,12 @@ constexpr int kXcorr3SmThreads = FFB_XCORR3_SM_THREADS;
 // ---------------------------------------------------------------------------
 // Row R2C (forward)
 // ---------------------------------------------------------------------------
+// Exchange groups of the row R2C: buffers 16 / FPB elements apart modulo a half-warp, as kBlockPad.
+template <int R, int P, int FPB>
+constexpr int kRowPad3 = (((FPB >= 16 ? 1 : FPB > 1 ? 16 / FPB : 0) - R * FftRShape<R, P>::SUB) % 16 + 16) % 16;
+template <int R, int P, int FPB>
+using RowGroup3 = FftRGroup<R, P, FPB, false, FftRShape<R, P>::SUB, kRowPad3<R, P, FPB>>;
+
 #ifndef FFB_ROWS3_MIN_BLOCKS
 #define FFB_ROWS3_MIN_BLOCKS 2
 #endif
@@ -45,7 +51,7 @@ r2c3_rows_kernel(RowFwdArgs a) {
     constexpr int T = S3::T;
     constexpr int TP = S3::TP;
     extern __shared__ float2 smem[];
-    using G = FftRGroup<R, P, FPB, false>;
+    using G = RowGroup3<R, P, FPB>;
     const int f = threadIdx.x / T;
     const int t = threadIdx.x - f * T;
     const int k2 = t / TP;

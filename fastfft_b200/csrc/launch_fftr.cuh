@@ -120,7 +120,7 @@ static cudaError_t r2c3_impl(const RowFwdArgs& a0, cudaStream_t st) {
     } else {
     constexpr int FPB = row_fpb3<R, P>();
     constexpr int THREADS = FftRShape<R, P>::T * FPB;
-    const size_t smem = (size_t)FftRGroup<R, P, FPB, false>::BYTES;
+    const size_t smem = (size_t)RowGroup3<R, P, FPB>::BYTES;
     RowFwdArgs a = a0;
     cudaError_t e = tables3(R, P, &a.tw, &a.tw3);
     if (e != cudaSuccess) return e;

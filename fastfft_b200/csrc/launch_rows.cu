@@ -8,7 +8,7 @@ template <int N, class InT>
 static cudaError_t r2c_impl(const RowFwdArgs& a, cudaStream_t st) {
     constexpr int FPB = r2c_fpb<N>();
     constexpr int THREADS = FftShape<N>::T * FPB;
-    const size_t smem = (size_t)FftGroup<N, FPB, false>::BYTES;
+    const size_t smem = (size_t)RowGroup<N, FPB>::BYTES;
     static std::atomic<unsigned long long> mask{0};
     auto fn = r2c_rows_kernel<N, InT, FPB>;
     cudaError_t e = ensure_smem_attr((const void*)fn, smem, &mask);
@@ -39,7 +39,7 @@ template <int N, class OutT>
 static cudaError_t c2r_impl(const RowInvArgs& a, cudaStream_t st) {
     constexpr int FPB = c2r_fpb<N>();
     constexpr int THREADS = FftShape<N>::T * FPB;
-    const size_t smem = (size_t)FftGroup<N, FPB, false>::BYTES;
+    const size_t smem = (size_t)RowGroup<N, FPB>::BYTES;
     static std::atomic<unsigned long long> mask{0};
     auto fn = c2r_rows_kernel<N, OutT, FPB>;
     cudaError_t e = ensure_smem_attr((const void*)fn, smem, &mask);
@@ -71,7 +71,7 @@ template <int N, class InC>
 static cudaError_t c2c_fwd_impl(const RowFwdArgs& a, cudaStream_t st) {
     constexpr int FPB = row_fpb<N>();
     constexpr int THREADS = FftShape<N>::T * FPB;
-    const size_t smem = (size_t)FftGroup<N, FPB, false>::BYTES;
+    const size_t smem = (size_t)RowGroup<N, FPB>::BYTES;
     static std::atomic<unsigned long long> mask{0};
     auto fn = c2c_rows_fwd_kernel<N, InC, FPB>;
     cudaError_t e = ensure_smem_attr((const void*)fn, smem, &mask);
@@ -101,7 +101,7 @@ template <int N, class OutC>
 static cudaError_t c2c_inv_impl(const RowInvArgs& a, cudaStream_t st) {
     constexpr int FPB = row_fpb<N>();
     constexpr int THREADS = FftShape<N>::T * FPB;
-    const size_t smem = (size_t)FftGroup<N, FPB, false>::BYTES;
+    const size_t smem = (size_t)RowGroup<N, FPB>::BYTES;
     static std::atomic<unsigned long long> mask{0};
     auto fn = c2c_rows_inv_kernel<N, OutC, FPB>;
     cudaError_t e = ensure_smem_attr((const void*)fn, smem, &mask);

@@ -85,12 +85,12 @@ struct FftRShape {
     // Region and FFT strides of the row C2R, which writes its input spectrum decimated by R
     // (Z[k] of FFT ff in region k % R at phys(k / R)); a warp's scatter covers consecutive k
     // of several FFTs.  For R = 3 the offsets past a multiple of 16 are the ones a bank model
-    // of that scatter finds best for the block shape of each P (at P = 512: 400 instead of
-    // 768 wavefronts per block); for R = 5 and 7 an odd region offset.  The sub-FFT exchanges read
+    // of that scatter finds best for the block shape of each P; for R = 5 and 7 an odd region
+    // offset.  The sub-FFT exchanges read
     // and write within one region and are conflict-free for any offset.
     static constexpr int C2R_SUB_EXTRA =
-        R != 3 ? 1 : P == 128 ? 5 : P == 256 ? 1 : P == 512 ? 3 : P == 1024 ? 3 : 11;
-    static constexpr int C2R_FFT_EXTRA = R != 3 ? 0 : P == 128 ? 0 : P == 256 ? 3 : P == 512 ? 3 : P == 1024 ? 15 : 0;
+        R != 3 ? 1 : P == 256 ? 1 : P == 1024 ? 3 : 11;
+    static constexpr int C2R_FFT_EXTRA = R != 3 ? 0 : P == 256 ? 3 : P == 1024 ? 15 : 0;
     static constexpr int SUB_C2R = (FftShape<P>::SMEM + 15) / 16 * 16 + C2R_SUB_EXTRA;
     static constexpr int SMEM = R * SUB;               // float2 per exchange buffer
     static constexpr int ROUNDS = (P + T - 1) / T;     // radix-R items per thread

@@ -8,6 +8,8 @@
 //   cols3_kernel       : column FFT (2D layout), forward / inverse / fused correlation, keep W
 //   xcorr3_cols_kernel : batched fused column pass (TMA-staged image and template columns,
 //                        forward, conj(T) * I, inverse), keep W
+// (The row passes at 384 and 1536 points and the batched pass at 384, 768 and 1536 run on the
+// split block FFT instead: kernels_rows_split.cuh, xcorr_split_kernel.)
 // Time-domain data are loaded and stored in natural order; the spectrum side is decimated
 // by R (thread (k2, j) holds X[R (j + T' q) + k2]).  R = 3 or 5 (lengths 3 * 2^k, 5 * 2^k).
 #pragma once
@@ -18,12 +20,10 @@
 namespace ffb {
 
 // Resident threads per SM the register budget of the column passes (batched and single) is
-// sized for: 480 (at most 136 registers; 128 used at 1536 points without spills), as 5 blocks
-// of one 1536-point FFT (96 threads) each.  Small blocks beat 2 blocks of 2 FFTs (named
-// barriers per FFT) on B200: 5.66 instead of 5.94 us per template at 1536 points in the
-// batched pass, 1.41 instead of 1.58 at 768.  Budgets measured side by side at 1536 points
-// (batched pass, us per template): 384 threads (156 registers, 4 blocks) 5.41-5.53, 480 (128
-// registers, 5 blocks) 5.12, 576 (96 registers, a few spills in other instantiations) 5.15-5.16.
+// sized for: 480 (at most 136 registers), in blocks of about 96 threads.  Small blocks beat 2
+// blocks of 2 FFTs (named barriers per FFT).  Measured with this form of the 1536-point batched
+// pass, which the split block FFT has replaced (kernels_xcorr.cuh): 384 threads (156 registers)
+// 5.41-5.53 us per template, 480 (128) 5.12, 576 (96, a few spills) 5.15-5.16.
 #ifndef FFB_XCORR3_SM_THREADS
 #define FFB_XCORR3_SM_THREADS 480
 #endif
@@ -118,11 +118,9 @@ r2c3_rows_kernel(RowFwdArgs a) {
 // Row C2R (inverse), optional fused peak search
 // ---------------------------------------------------------------------------
 // The C2R gathers its input from L2/HBM with all of a thread's loads in flight at once, so it
-// gains from a third resident block per SM (56 registers; measured on B200 at 1536 points:
-// 4.2 instead of 4.6 us per template); the R2C does not, and keeps two.  Measured again with
-// the 1536-point step (us per template): R2C at 3 blocks (56 registers, 48 bytes spilled)
-// 2.086 against 2.093 at 2, within noise; C2R at 4 blocks (40 registers, 104 bytes spilled)
-// 3.96 against 2.81 at 3.
+// gains from a third resident block per SM (56 registers; measured on B200 with this form of the
+// 1536-point pass: 4.2 instead of 4.6 us per template; at 4 blocks, 40 registers and spills, 3.96
+// against 2.81 at 3); the R2C does not (2.086 against 2.093), and keeps two.
 #ifndef FFB_C2R3_MIN_BLOCKS
 #define FFB_C2R3_MIN_BLOCKS 3
 #endif
@@ -351,9 +349,8 @@ cols3_kernel(ColArgs a) {
 // Batched fused correlation column pass (as xcorr_cols_kernel)
 // ---------------------------------------------------------------------------
 // One exchange buffer per FFT: the sub-FFT exchanges synchronise one warp (P = 512) or
-// their own T' threads, so double buffering saves little, while the 26 KB it costs at
-// P = 512 decides whether two blocks fit on an SM with 16 templates staged (measured on
-// B200: 8.5 instead of 9.4 us per template for the 1536-point pass).
+// their own T' threads, so double buffering saves little, while its shared memory decides how
+// many blocks with staged templates fit on an SM.
 constexpr bool kXcorr3DB = false;
 
 template <int R, int P, class ImgC, int FPB>
@@ -424,8 +421,7 @@ xcorr3_cols_kernel(XcorrColArgs a) {
         float2 v[16];
         const float2* src = t1_s + (live ? gl : 0) * lcol;
         // Templates that end before P (the usual case: L + W - 1 <= 3P with W >= L) need
-        // only x[n1]; this block-uniform branch skips the other two loads and the radix-3
-        // sums (measured on B200 at 1536 points: 7.2 instead of 7.8 us per template).
+        // only x[n1]; this block-uniform branch skips the other loads and the radix-R sums.
         if (Lg <= P) {
             // y_k2[n1] = W_3P^(n1 k2) x[n1]
 #pragma unroll

@@ -1,6 +1,8 @@
-// Fused cross-correlation column pass, batched over templates (sm_100a).
-//
-// One block per spectrum column kx serves every template of the batch:
+// Fused cross-correlation column pass, batched over templates (sm_100a), in two forms:
+// xcorr_split_kernel (below) at the lengths of the split block FFT (256 ... 2048 and 384 ... 1536),
+// where it replaced the first one, and xcorr_cols_kernel at the other powers of two (16 ... 128,
+// 4096; the other R * 2^k lengths are in kernels_fft3.cuh).  In the latter, one block per spectrum
+// column kx serves the templates of a group:
 //   - the image-spectrum column (N values) and the template row-pass columns (L values
 //     per template) are brought into shared memory by TMA bulk copies
 //     (cp.async.bulk ... mbarrier::complete_tx) issued by one thread, so the image
@@ -61,12 +63,8 @@ struct XcorrSmem {
     static __host__ __device__ constexpr int total(int L, int nb) { return bar_off(L, nb) + 16; }
 };
 
-// Block size of the batched column pass: 128 threads (several FFTs per block below N = 2048),
-// with registers budgeted for 512 resident threads per SM.  Smaller blocks than the former 256
-// threads measured faster on B200: 2.06 instead of 2.18 us per template at 1024^2, 0.23
-// instead of 0.32 at 256^2 (64 per launch).  Budgets of 640 (92 registers at 1024) and 768
-// (80) measured on the uneven batch: 383,887-387,140 and 373,363-373,437 templates/s against
-// 385,195-385,889 with 512.
+// Block size of xcorr_cols_kernel: 128 threads (one FFT from N = 2048 up), with registers budgeted
+// for 512 resident threads per SM.
 constexpr int kXcorrBlockThreads = 128;
 #ifndef FFB_XCORR_SM_THREADS
 #define FFB_XCORR_SM_THREADS 512

@@ -29,9 +29,8 @@ namespace ffb {
 
 // FFTs per block: up to 384 threads for the row passes and 256 for the column passes, in
 // whole warps (the peak search shuffles over full warps).  Row blocks of 384 threads hold a
-// power-of-two number of FFTs (4 at 1536 points), whose buffers the gather and split phases
-// interleave without bank conflicts (5 FFTs of 96 threads cost 47 % extra shared-memory
-// wavefronts there); measured on B200: 15.6 instead of 15.8 us per template at 1536^2.
+// power-of-two number of FFTs at R = 3, whose buffers the gather and split phases interleave
+// without bank conflicts.
 // (the most FFTs up to the target whose threads fill whole warps; if none does, the fewest
 // above it that do, e.g. 4 FFTs of 40 threads at length 640)
 constexpr int fpb3_for(int t, int target) {
@@ -45,9 +44,7 @@ template <int R, int P>
 constexpr int row_fpb3() {
     return fpb3_for(FftRShape<R, P>::T, 384);
 }
-// column passes: blocks of about 96 threads (one FFT from P = 512 up), as the batched pass;
-// measured on B200 in the image preparation of the 384^2 -> 4096^2 -> 1024^2 step: 647.7
-// instead of 650.3 us per step with the 1536-point forward columns in 192-thread blocks
+// column passes: blocks of about 96 threads (one FFT from P = 512 up), as the batched pass
 template <int R, int P>
 constexpr int col_fpb3() {
     return fpb3_for(FftRShape<R, P>::T, 96);

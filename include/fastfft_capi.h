@@ -196,7 +196,7 @@ FASTFFT_API fastfft_status fastfft_set_templates_per_launch(fastfft_handle h, in
 FASTFFT_API fastfft_status fastfft_templates_per_launch(fastfft_handle h, int* n);
 
 /* Templates that one block of the batched fused column pass stages and transforms (0, the
- * default: a per-length choice measured on B200 -- 6 at length 1536, 4 at 1024, 8 elsewhere),
+ * default: a choice by length and templates per launch measured on B200, 4 to 12),
  * and the value in effect for the plan's correlation size.  No reference counterpart. */
 FASTFFT_API fastfft_status fastfft_set_templates_per_block(fastfft_handle h, int n);
 FASTFFT_API fastfft_status fastfft_templates_per_block(fastfft_handle h, int* n);

@@ -175,8 +175,8 @@ __device__ __forceinline__ float2 c_part(cpair v, int w) {
 }
 
 // Shared memory of a block: the image column, stored as P rows of E values (frequency s + E kp
-// at row kp) of a stride that keeps the reads at freq_index free of bank conflicts, the exchange buffers of the G groups, and the input columns that each group works on
-// next, thread by thread.
+// at row kp) of a stride that keeps the reads at freq_index free of bank conflicts, the exchange
+// buffers of the G groups, and the input columns that each group works on next, thread by thread.
 template <int N, class C, int G>
 struct XcorrSplitSmem {
     using F = SplitFft<N, C>;

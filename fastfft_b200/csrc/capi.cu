@@ -1070,7 +1070,19 @@ static fastfft_status red_xcorr_batch(fastfft_handle h, int mx, int my, int n, c
     std::memset(&a, 0, sizeof(a));
     for (int g = 0; g < n; g++) a.in[g] = inputs[g];
     a.n_batch = n;
-    a.in_pitch = 2LL * h->fwd_in.w; a.n_rows = (int)h->fwd_in.y; a.L = (int)h->fwd_in.x;
+    // the largest template of this group, which in an uneven batch can be far smaller than the
+    // plan's (and the plan's taller than the group's length my): the row pass starts no blocks, and
+    // the column pass stages nothing, for rows that no template here has (768-point groups of
+    // templates up to 256 rows under a plan of 384: four blocks per SM instead of three)
+    int lx = (int)h->fwd_in.x, ly = (int)h->fwd_in.y;
+    if (dims) {
+        lx = ly = 0;
+        for (int g = 0; g < n; g++) {
+            lx = std::max(lx, dims[2 * g]);
+            ly = std::max(ly, dims[2 * g + 1]);
+        }
+    }
+    a.in_pitch = 2LL * h->fwd_in.w; a.n_rows = ly; a.L = lx;
     a.out = t1; a.out_pitch = h->pitch_a; a.out_batch_stride = h->red_t1_stride;
     a.kmax = mx / 2 + 1; a.scale = scale_of(pre_op); a.tw = tw;
     if (dims) {
@@ -1089,7 +1101,7 @@ static fastfft_status red_xcorr_batch(fastfft_handle h, int mx, int my, int n, c
     if ((e = twiddles_for(my, &tw)) != cudaSuccess) return cuda_fail(h, e, "twiddle table");
     XcorrColArgs c;
     std::memset(&c, 0, sizeof(c));
-    c.t1 = t1; c.t1_pitch = h->pitch_a; c.t1_batch = h->red_t1_stride; c.L = (int)h->fwd_in.y;
+    c.t1 = t1; c.t1_pitch = h->pitch_a; c.t1_batch = h->red_t1_stride; c.L = ly;
     c.img = spec; c.img_stride = my;
     c.out = t2; c.out_pitch = h->pitch_b; c.out_batch = h->red_t2_stride; c.W = (int)h->inv_out.y;
     c.n_cols = mx / 2 + 1; c.n_batch = n;
@@ -1099,7 +1111,8 @@ static fastfft_status red_xcorr_batch(fastfft_handle h, int mx, int my, int n, c
     c.intra_kind = intra_op ? intra_op->kind : FASTFFT_OP_NOOP;
     c.intra_scale = intra_op ? intra_op->scale : 1.f;
     c.tw = tw; c.err = h->dev_err;
-    c.tc = h->tc_dft ? 1 : 0;
+    // (by the plan's height, as fastfft_tensor_core_dft_active reports it)
+    c.tc = h->tc_dft && h->fwd_in.y <= 512 ? 1 : 0;
     if ((e = launch_xcorr_cols(my, FASTFFT_DTYPE_C64, c, h->stream)) != cudaSuccess)
         return cuda_fail(h, e, "cross-correlation column pass");
     h->launches++;

@@ -61,3 +61,60 @@ def test_split_lengths(torch_cuda, m, n, tmpl, win):
     for other in results[1:]:
         for a, b in zip(results[0], other):
             assert np.array_equal(a, b)
+
+
+# (class, transform height, plan's template height, template height of the class, window height):
+# the plan's templates are taller than the whole class is long
+TALL_PLANS = [
+    (256, 1024, 384, 100, 100),
+    (384, 1024, 450, 150, 180),
+    (512, 2048, 600, 200, 250),
+    (768, 2048, 800, 250, 500),
+    (1024, 3072, 1100, 300, 600),
+    (1536, 4096, 1600, 500, 1000),
+]
+
+
+@pytest.mark.parametrize("m,ny,tall,small,wy", TALL_PLANS)
+def test_plan_taller_than_a_class(torch_cuda, m, ny, tall, small, wy):
+    """Uneven batches whose shorter templates correlate at a length below the plan's template
+    height: windows against the oracle; peaks and projection against those windows."""
+    import torch
+
+    import fastfft_b200 as F
+    from oracle import fastfft_oracle as O
+
+    rng = np.random.default_rng(m)
+    nx, tx, wx = 512, 60, 61
+    fout, iout = (nx, ny, 1), (wx, wy, 1)
+    assert m // 2 < small + wy - 1 <= m < tall
+    spec = O.fwd(O.real_to_padded(rng.standard_normal((ny, nx)), fout, dtype=np.float64), fout, fout)
+    spec = (spec / np.sqrt(nx * ny)).astype(np.complex64)
+    ft = F.FourierTransformer()
+    ft.SetForwardFFTPlan(tx, tall, 1, *fout)
+    ft.SetInverseFFTPlan(*fout, *iout)
+    sizes = [(tx, small), (tx, tall), (41, small - 3), (tx, small), (23, small), (tx - 1, tall - 1)]
+    ts = [rng.standard_normal((y, x)).astype(np.float32) for x, y in sizes]
+    ins = [torch.from_numpy(O.real_to_padded(t, (x, y, 1))).cuda() for t, (x, y) in zip(ts, sizes)]
+    d_spec = torch.from_numpy(spec.view(np.float32).reshape(-1).copy()).cuda()
+    size = ft.ReturnInvOutputMemorySize()
+    outs, outs2 = ([torch.zeros(size, device="cuda") for _ in ts] for _ in range(2))
+    peaks = torch.zeros(len(ts), dtype=torch.int64, device="cuda")
+    mip = torch.zeros(wx * wy, dtype=torch.int64, device="cuda")
+    ft.FwdImageInvFFTManySized(ins, sizes, d_spec, outs)
+    ft.FwdImageInvFFTManyPeaks(ins, d_spec, peaks, sizes=sizes, outputs=outs2)
+    ft.FwdImageInvFFTManyMip(ins, d_spec, mip, sizes=sizes)
+    wins = np.stack([O.real_from_padded(o.cpu().numpy(), iout)[0] for o in outs])
+    for t, (x, y), got in zip(ts, sizes, wins):
+        plan = O.Plan((x, y, 1), fout, fout, iout)
+        ref = O.real_from_padded(
+            O.fwd_image_inv(O.real_to_padded(t, (x, y, 1)), spec, plan, out_dtype=np.float64), iout)[0]
+        assert O.rel_l2(got, ref) <= RTOL_L2_FP32, (x, y)
+        assert O.rel_max(got, ref) <= RTOL_MAX_FP32, (x, y)
+    for a, b in zip(outs, outs2):
+        assert torch.equal(a, b)
+    vals, idx = F.decode_peaks(peaks)
+    flat = wins.reshape(len(ts), -1)
+    assert np.array_equal(idx, flat.argmax(1)) and np.array_equal(vals, flat.max(1))
+    vals, idx = F.decode_peaks(mip)
+    assert np.array_equal(idx, flat.argmax(0)) and np.array_equal(vals, flat.max(0))

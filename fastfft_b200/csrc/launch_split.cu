@@ -15,6 +15,13 @@ static cudaError_t xcorr_split_impl(const XcorrColArgs& a, cudaStream_t st) {
     return launch_dependent(fn, dim3(a.n_cols, (a.n_batch + a.tpb - 1) / a.tpb), SplitFft<N, C>::T * G, smem, st, a);
 }
 
+// Whether three blocks of the pair, its occupancy by registers, fit on an SM at template height L
+// (228 KB of shared memory, 1 KB of it per block kept by the system).
+template <int N, int G>
+static bool pair_fits(int L) {
+    return 3 * (XcorrSplitSmem<N, cpair, G>::total(L) + 1024) <= 228 * 1024;
+}
+
 // Blocks of G transform groups; registers for MIN_BLOCKS blocks per SM.  Measured on B200 (us per
 // launch; "before": the radix-16 forms xcorr_cols_kernel / xcorr3_cols_kernel, which keep the
 // other lengths):
@@ -30,7 +37,17 @@ static cudaError_t xcorr_split_impl(const XcorrColArgs& a, cudaStream_t st) {
 //   2048 (500, 1100, 16)                     159    136 (1 x 4)    129 (1 x 3)
 // The single form at 128 registers (16 warps per SM) is the better one at most lengths (at 96 it
 // spills: 382 us at 1536); at 2048, and at 1536 once a launch holds 16 templates, the pair is (168
-// registers, 12 warps).  Fewer than four templates take blocks of one group, so that no group
+// registers, 12 warps), while its staged columns leave room for three blocks: up to 448 template
+// rows at 1536 and 1600 at 2048.  Above, two blocks (8 warps) are the slower form (us per launch, pair
+// / single, same length and launch size, the window filling the length; both are flat on either
+// side of the line):
+//   1536, L = 448:  80.6 / 82.3 (16 templates)  153.8 / 154.5 (32)  282 / 295 (64)
+//   1536, L = 449:  91.7 / 82.2                 171.1 / 155.0       325 / 295
+//   1536, L = 1000: 92.5 / 86.0                 173.6 / 161.7       330 / 308
+//   2048, L = 1000: 135.2 / 138.3 (16)          258 / 264 (32)
+//   2048, L = 1590: 144.5 / 142.0               277 / 273
+//   2048, L = 1610: 159.2 / 142.7               305 / 273
+// Fewer than four templates take blocks of one group, so that no group
 // idles.  At 1536 the pair's launch keeps the FP32 pipe 53 %, the shared-memory path 65 % and the
 // issue slots 57 % busy at 3 warps per scheduler: bound by latency at that occupancy (before: 48,
 // 75 and 71 %).  Both forms give the same bits (cpair.cuh), so the choice does not show in results.
@@ -53,10 +70,10 @@ cudaError_t launch_xcorr_split(int n, const XcorrColArgs& a0, cudaStream_t st) {
             return xcorr_split_impl<1024, float2, 2, 4>(a, st);
         case 1536:
             if (few) return xcorr_split_impl<1536, float2, 1, 8>(a, st);
-            if (a.n_batch < 16) return xcorr_split_impl<1536, float2, 2, 4>(a, st);
-            return xcorr_split_impl<1536, cpair, 2, 3>(a, st);
+            if (a.n_batch >= 16 && pair_fits<1536, 2>(a.L)) return xcorr_split_impl<1536, cpair, 2, 3>(a, st);
+            return xcorr_split_impl<1536, float2, 2, 4>(a, st);
         case 2048:
-            if (few) return xcorr_split_impl<2048, float2, 1, 4>(a, st);
+            if (few || !pair_fits<2048, 1>(a.L)) return xcorr_split_impl<2048, float2, 1, 4>(a, st);
             return xcorr_split_impl<2048, cpair, 1, 3>(a, st);
         default: return cudaErrorInvalidValue;
     }

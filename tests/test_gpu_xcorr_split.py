@@ -22,6 +22,11 @@ CASES = [
     (1536, 2048, (384, 384), (1024, 1023)),
     (1536, 2048, (300, 901), (900, 600)),
     (2048, 3072, (512, 513), (1200, 1300)),
+    # the last template heights whose pairs fit three blocks on an SM, and the first that do not
+    (1536, 2048, (60, 448), (100, 1089)),
+    (1536, 2048, (60, 449), (100, 1088)),
+    (2048, 3072, (60, 1600), (100, 449)),
+    (2048, 3072, (60, 1601), (100, 448)),
 ]
 
 

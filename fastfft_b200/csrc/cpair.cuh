@@ -195,18 +195,33 @@ constexpr int pfa_in(int n3, int n8) { return (8 * n3 + 3 * n8) % 24; }
 constexpr int pfa_out(int k3, int k8) { return (16 * k3 + 9 * k8) % 24; }  // 16 = (1, 0), 9 = (0, 1) mod (3, 8)
 
 template <bool INV, class C>
-__device__ __forceinline__ void pdft24(C (&v)[24]) {
+__device__ __forceinline__ void pdft24_eights(C (&v)[24]) {
 #pragma unroll
     for (int a = 0; a < 3; a++)
         pdft8<INV>(v[pfa_in(a, 0)], v[pfa_in(a, 1)], v[pfa_in(a, 2)], v[pfa_in(a, 3)], v[pfa_in(a, 4)],
                    v[pfa_in(a, 5)], v[pfa_in(a, 6)], v[pfa_in(a, 7)]);
+}
+template <bool INV, class C>
+__device__ __forceinline__ void pdft24_threes(C (&v)[24]) {
+#pragma unroll
+    for (int b = 0; b < 8; b++) pdft3<INV>(v[pfa_in(0, b)], v[pfa_in(1, b)], v[pfa_in(2, b)]);
+}
+// The forward DFT24 takes the DFT3s first, as its short head below does, so that both give the
+// same bits where the short one applies: which of the two a pair takes depends on both its templates.
+template <bool INV, class C>
+__device__ __forceinline__ void pdft24(C (&v)[24]) {
+    if constexpr (INV) {
+        pdft24_eights<INV>(v);
+        pdft24_threes<INV>(v);
+    } else {
+        pdft24_threes<INV>(v);
+        pdft24_eights<INV>(v);
+    }
     C t[24];
 #pragma unroll
-    for (int b = 0; b < 8; b++) {
-        pdft3<INV>(v[pfa_in(0, b)], v[pfa_in(1, b)], v[pfa_in(2, b)]);
+    for (int a = 0; a < 3; a++)
 #pragma unroll
-        for (int a = 0; a < 3; a++) t[pfa_out(a, b)] = v[pfa_in(a, b)];
-    }
+        for (int b = 0; b < 8; b++) t[pfa_out(a, b)] = v[pfa_in(a, b)];
 #pragma unroll
     for (int k = 0; k < 24; k++) v[k] = t[k];
 }

@@ -68,6 +68,46 @@ def test_split_lengths(torch_cuda, m, n, tmpl, win):
             assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("m,ny,tall,short,wy", [(1536, 2048, 448, 1, 1089), (2048, 3072, 1000, 489, 1049)])
+def test_pairs_of_unequal_height(torch_cuda, m, ny, tall, short, wy):
+    """17 templates of different heights in one launch of the paired form: windows against the
+    oracle, and bit for bit as launches of one template give them."""
+    import torch
+
+    import fastfft_b200 as F
+    from oracle import fastfft_oracle as O
+
+    rng = np.random.default_rng(m + 1)
+    nx, tx, wx = 512, 60, 61
+    fout, iout = (nx, ny, 1), (wx, wy, 1)
+    spec = O.fwd(O.real_to_padded(rng.standard_normal((ny, nx)), fout, dtype=np.float64), fout, fout)
+    spec = (spec / np.sqrt(nx * ny)).astype(np.complex64)
+    heights = [tall, short, short, tall, tall - 1, short + 1] + [int(h) for h in rng.integers(short, tall + 1, 11)]
+    sizes = [(tx - k % 3, h) for k, h in enumerate(heights)]
+    ts = [rng.standard_normal((y, x)).astype(np.float32) for x, y in sizes]
+    ins = [torch.from_numpy(O.real_to_padded(t, (x, y, 1))).cuda() for t, (x, y) in zip(ts, sizes)]
+    d_spec = torch.from_numpy(spec.view(np.float32).reshape(-1).copy()).cuda()
+    ft = F.FourierTransformer()
+    ft.SetForwardFFTPlan(tx, tall, 1, *fout)
+    ft.SetInverseFFTPlan(*fout, *iout)
+    assert ft.CorrelationSize()[1] == m
+    results = []
+    for per_launch in (17, 1):
+        ft.SetTemplatesPerLaunch(per_launch)
+        outs = [torch.zeros(ft.ReturnInvOutputMemorySize(), device="cuda") for _ in ts]
+        before = ft.LaunchCount()
+        ft.FwdImageInvFFTManySized(ins, sizes, d_spec, outs)
+        assert ft.LaunchCount() - before == 4 + 3 * (17 // per_launch)   # one class: one preparation
+        results.append([O.real_from_padded(o.cpu().numpy(), iout) for o in outs])
+    for t, (x, y), got, alone in zip(ts, sizes, *results):
+        plan = O.Plan((x, y, 1), fout, fout, iout)
+        ref = O.real_from_padded(
+            O.fwd_image_inv(O.real_to_padded(t, (x, y, 1)), spec, plan, out_dtype=np.float64), iout)
+        assert O.rel_l2(got, ref) <= RTOL_L2_FP32, (x, y)
+        assert O.rel_max(got, ref) <= RTOL_MAX_FP32, (x, y)
+        assert np.array_equal(got, alone), (x, y)
+
+
 # (class, transform height, plan's template height, template height of the class, window height):
 # the plan's templates are taller than the whole class is long
 TALL_PLANS = [

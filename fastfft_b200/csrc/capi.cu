@@ -263,16 +263,18 @@ void size_buffers(fastfft_plan_s* h) {
             const long long spec = (mx / 2 + 1) * my * 8;                                // reduced spectrum
             h->off_c_real = round_up(stage, 256);
             h->off_c_spec = h->off_c_real + round_up(real, 256);
-            // templates per launch: bounded by the shared memory of the fused column kernel
+            // templates per launch: bounded by the shared memory of the fused column kernel where
+            // its blocks stage all their templates; the split form stages them per round and fits
+            // at any setting (asserted at its launcher)
             h->red_batch = h->red_batch_request;
-            while (h->red_batch > 1 &&
-                   xcorr_cols_smem((int)my, FASTFFT_DTYPE_C64, (int)h->fwd_in.y, xcorr_tpb(h, h->red_batch, my)) >
-                       226 * 1024)
-                h->red_batch--;
-            if (xcorr_cols_smem((int)my, FASTFFT_DTYPE_C64, (int)h->fwd_in.y, 1) > 226 * 1024) {
-                h->red_ok = false;
-                h->bytes_c = 0;
-                return;
+            if (!ffb::is_split_size((int)my)) {
+                auto smem = [&](int tpb) { return xcorr_cols_smem((int)my, FASTFFT_DTYPE_C64, (int)h->fwd_in.y, tpb); };
+                while (h->red_batch > 1 && smem(xcorr_tpb(h, h->red_batch, my)) > 226 * 1024) h->red_batch--;
+                if (smem(1) > 226 * 1024) {
+                    h->red_ok = false;
+                    h->bytes_c = 0;
+                    return;
+                }
             }
             h->red_t1_stride = round_up((mx / 2 + 1) * h->pitch_a, 32);   // complex elements per template
             h->red_t2_stride = round_up((mx / 2 + 1) * h->pitch_b, 32);   // column output [kx][y]

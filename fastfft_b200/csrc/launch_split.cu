@@ -7,6 +7,7 @@ namespace ffb {
 
 template <int N, class C, int G, int MIN_BLOCKS>
 static cudaError_t xcorr_split_impl(const XcorrColArgs& a, cudaStream_t st) {
+    static_assert(XcorrSplitSmem<N, C, G>::total(N) <= 227 * 1024, "fits for every template height");
     const int smem = XcorrSplitSmem<N, C, G>::total(a.L);
     static std::atomic<int> high_water[64];
     auto fn = xcorr_split_kernel<N, C, G, MIN_BLOCKS>;

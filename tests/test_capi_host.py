@@ -219,3 +219,21 @@ def test_chirp_z_lengths_complex_and_3d():
         with pytest.raises(F.FastFFTError) as e:
             ft.SetInverseFFTPlan(*fout, *fout)
         assert e.value.status == C.ERR_INVALID_DIMS
+
+
+def test_templates_per_launch_bound_follows_the_column_kernel():
+    """The split column pass stages per round, so its launches hold the requested templates whatever
+    the templates per block; the staged form at 4096 points holds what fits in shared memory."""
+    for fin, fout, iout, full in (((384, 384, 1), (2048, 2048, 1), (1024, 1024, 1), True),
+                                  ((300, 900, 1), (4096, 4096, 1), (400, 1100, 1), True),
+                                  ((300, 1500, 1), (4096, 8192, 1), (400, 2500, 1), False)):
+        ft = new()
+        ft.SetTemplatesPerLaunch(64)
+        ft.SetForwardFFTPlan(*fin, *fout)
+        ft.SetInverseFFTPlan(*fout, *iout)
+        assert ft.TemplatesPerLaunch() == 64
+        ft.SetTemplatesPerBlock(64)
+        assert (ft.TemplatesPerLaunch() == 64) == full
+        assert ft.TemplatesPerBlock() == ft.TemplatesPerLaunch()
+        ft.SetTemplatesPerBlock(0)
+        assert ft.TemplatesPerLaunch() == 64

@@ -51,7 +51,17 @@ class KernelFunction:
         return C.fastfft_op(C.OP_CONJ_MUL_THEN_SCALE, float(s))
 
 
-_torch = None   # the torch module, once a plan has been bound to one of its streams
+_raw_stream_of = None   # raw handle of torch's current stream, once torch and its CUDA state are up
+
+
+def _raw_stream_call(torch):
+    """A call that returns the raw handle of the current stream: torch's own raw-handle functions (not a
+    public interface; the public call builds a Stream object, about 5 us of a 13 us transform), or
+    the public call if this torch does not have them."""
+    raw, device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
 
 
 def _ptr(x) -> int | None:
@@ -132,23 +142,21 @@ class FourierTransformer:
             raise C.FastFFTError(st, self._lib.fastfft_last_error(self._h).decode())
 
     def _bind_stream(self):
-        global _torch
+        global _raw_stream_of
         if self._stream is not None:
             return
-        if self._raw_stream is not None:
-            # torch and its CUDA state are up: the raw handle of the current stream, which the
-            # plan is told only when it changes (about 5 us of a 13 us call otherwise)
-            raw = _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
-            if raw == self._raw_stream:
-                return
-        else:
+        if _raw_stream_of is None:
             try:
-                import torch as _torch
+                import torch
             except ImportError:  # pragma: no cover - torch is part of the image
                 return
-            if not _torch.cuda.is_available():
+            if not torch.cuda.is_available():
                 return
-            raw = _torch.cuda.current_stream().cuda_stream
+            torch.cuda.current_stream()   # (brings up torch's CUDA state, which the raw calls need)
+            _raw_stream_of = _raw_stream_call(torch)
+        raw = _raw_stream_of()
+        if raw == self._raw_stream:   # the plan is told only when it changes
+            return
         self._check(self._lib.fastfft_set_stream(self._h, raw))
         self._raw_stream = raw
 

@@ -237,3 +237,29 @@ def test_templates_per_launch_bound_follows_the_column_kernel():
         assert ft.TemplatesPerBlock() == ft.TemplatesPerLaunch()
         ft.SetTemplatesPerBlock(0)
         assert ft.TemplatesPerLaunch() == 64
+
+
+@pytest.mark.parametrize("fast", [False, True])
+def test_plan_follows_torch_streams(monkeypatch, fast):
+    """The plan is told torch's current stream when it changes, through torch's raw-handle calls where
+    they exist and the public one otherwise."""
+    import sys
+    import types
+
+    from fastfft_b200 import transformer
+
+    now = types.SimpleNamespace(cuda_stream=0x100)
+    fake = types.SimpleNamespace(
+        cuda=types.SimpleNamespace(is_available=lambda: True, current_stream=lambda: now),
+        _C=types.SimpleNamespace(**({"_cuda_getCurrentRawStream": lambda device: now.cuda_stream + device,
+                                     "_cuda_getDevice": lambda: 0} if fast else {})))
+    monkeypatch.setitem(sys.modules, "torch", fake)
+    monkeypatch.setattr(transformer, "_raw_stream_of", None, raising=False)
+    told = []
+    ft = new()
+    ft._lib = types.SimpleNamespace(fastfft_set_stream=lambda h, s: told.append(s) or C.OK)
+    for raw in (0x100, 0x100, 0x200, 0, 0, 0x100):
+        now.cuda_stream = raw
+        ft._bind_stream()
+    assert told == [0x100, 0x200, 0, 0x100]
+    ft._lib = C.lib()

@@ -73,20 +73,17 @@ template <int A, int B, int BYTES>
 struct SplitLayout {
     static constexpr int P = A * B;
     static constexpr int LANES = 128 / BYTES;                    // elements per wavefront
-    static constexpr bool XOR_ROW = B >= 8;                      // i ^ row
-    static constexpr bool XOR_4 = B == 4 && LANES == 8;
-    static constexpr bool SWIZZLE = XOR_ROW || XOR_4;
+    static constexpr bool SWIZZLE = B >= 8;                      // i ^ row
     static constexpr int PS = SWIZZLE || B == 1 ? B : B + 1;     // stride of k1 in the exchange
     static constexpr int NEED = A * PS > P ? A * PS : P;
     // padded regions of consecutive sub-FFTs start B elements apart modulo a wavefront
     static constexpr int RS = SWIZZLE ? P : NEED + ((B - NEED) % LANES + LANES) % LANES;
     static constexpr int MASK = (B < LANES ? B : LANES) - 1;
     // the parity of the sub-FFT moves it to the other half of a wavefront
-    static constexpr int PAR = XOR_4 ? 6 : (XOR_ROW && B < LANES) ? B : 0;
+    static constexpr int PAR = SWIZZLE && B < LANES ? B : 0;
     static __device__ __forceinline__ int nat(int b, int p) { return PAR ? b ^ (p ? PAR : 0) : b; }
     static __device__ __forceinline__ int ex(int k1, int i, int p) {
-        if constexpr (XOR_ROW) return (k1 * B + (i ^ (k1 & MASK))) ^ (PAR && p ? PAR : 0);
-        else if constexpr (XOR_4) return (k1 * B + (i ^ ((k1 >> 1) & 3))) ^ (p ? PAR : 0);
+        if constexpr (SWIZZLE) return (k1 * B + (i ^ (k1 & MASK))) ^ (PAR && p ? PAR : 0);
         else return k1 * PS + i;
     }
 };

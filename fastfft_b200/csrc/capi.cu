@@ -1103,7 +1103,13 @@ static fastfft_status red_xcorr_batch(fastfft_handle h, int mx, int my, int n, c
     if ((e = twiddles_for(my, &tw)) != cudaSuccess) return cuda_fail(h, e, "twiddle table");
     XcorrColArgs c;
     std::memset(&c, 0, sizeof(c));
-    c.t1 = t1; c.t1_pitch = h->pitch_a; c.t1_batch = h->red_t1_stride; c.L = ly;
+    c.t1 = t1; c.t1_pitch = h->pitch_a; c.t1_batch = h->red_t1_stride;
+    // Two groups in flight stage by the plan's height: the three blocks per SM of the case above leave
+    // registers for the other group's row passes, which four do not (1024 templates of 128 ... 384 in
+    // one graph, ms by the group's / the plan's height: one group of 64 2.449 / 2.478, two of 32
+    // 2.377 / 2.340).
+    const bool two_groups = h->pipe_groups > 1 && h->pipe_stream;
+    c.L = two_groups ? std::min((int)h->fwd_in.y, my) : ly;
     c.img = spec; c.img_stride = my;
     c.out = t2; c.out_pitch = h->pitch_b; c.out_batch = h->red_t2_stride; c.W = (int)h->inv_out.y;
     c.n_cols = mx / 2 + 1; c.n_batch = n;

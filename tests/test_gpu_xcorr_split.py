@@ -120,10 +120,12 @@ TALL_PLANS = [
 ]
 
 
+@pytest.mark.parametrize("groups", [1, 2])
 @pytest.mark.parametrize("m,ny,tall,small,wy", TALL_PLANS)
-def test_plan_taller_than_a_class(torch_cuda, m, ny, tall, small, wy):
+def test_plan_taller_than_a_class(torch_cuda, m, ny, tall, small, wy, groups):
     """Uneven batches whose shorter templates correlate at a length below the plan's template
-    height: windows against the oracle; peaks and projection against those windows."""
+    height, one or two groups in flight: windows against the oracle; peaks and projection against
+    those windows."""
     import torch
 
     import fastfft_b200 as F
@@ -136,8 +138,11 @@ def test_plan_taller_than_a_class(torch_cuda, m, ny, tall, small, wy):
     spec = O.fwd(O.real_to_padded(rng.standard_normal((ny, nx)), fout, dtype=np.float64), fout, fout)
     spec = (spec / np.sqrt(nx * ny)).astype(np.complex64)
     ft = F.FourierTransformer()
+    ft.SetTemplatesPerLaunch(16 if groups == 1 else 2)
+    ft.SetPipelinedGroups(groups)
     ft.SetForwardFFTPlan(tx, tall, 1, *fout)
     ft.SetInverseFFTPlan(*fout, *iout)
+    assert ft.PipelinedGroups() == groups
     sizes = [(tx, small), (tx, tall), (41, small - 3), (tx, small), (23, small), (tx - 1, tall - 1)]
     ts = [rng.standard_normal((y, x)).astype(np.float32) for x, y in sizes]
     ins = [torch.from_numpy(O.real_to_padded(t, (x, y, 1))).cuda() for t, (x, y) in zip(ts, sizes)]

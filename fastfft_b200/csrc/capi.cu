@@ -27,19 +27,17 @@
 
 using namespace ffb;
 
-// Templates per block of the fused column pass (0: the whole launch's group).  Splitting a
-// group of 16 over two blocks per column doubles the blocks of a launch (1538 instead of 769
-// at 1536^2, 5.2 instead of 2.6 waves of two blocks per SM), which shortens the last, partly
-// empty wave; the image column is then staged twice, from L2.  Measured on B200 at 16
-// templates per launch: 7.8 instead of 8.5 us per template at 1536^2, 2.9 instead of 3.7 at
-// 1024^2.
+// Templates per block of the fused column pass where xcorr_tpb below makes no choice of its own (0:
+// the whole launch's group).  Fewer per block give more blocks and a shorter last, partly empty wave;
+// the image column is then staged by more blocks, from L2.
 #ifndef FFB_XCORR_TPB
 #define FFB_XCORR_TPB 8
 #endif
 
 // templates that one block of the fused column pass serves for a launch of n at column length
-// my; measured best on B200: at 1536 twelve from 16 templates up (266 us per 64-template launch;
-// 282 - 300 with the tensor-core and three-group forms' 6) and six below, at 384 four up to 16
+// my; measured best on B200: at 1536 twelve from 16 templates up (265 us per 64-template launch;
+// 279 with eight, 283 with four, 347 with six) and six below (the single form: 65 us at 12 templates,
+// 72 with twelve), at 384 four up to 16
 // templates (10.0 instead of 14.3 us at 12) and eight above, eight elsewhere (at 1024: 66.1 us
 // per 32 templates; 68.7 with four or six, 70.6 with twelve)
 // (fastfft_set_templates_per_block overrides it; the autotuner measures the candidates)

@@ -2,10 +2,12 @@
 // block FFT (fft_split.cuh) is written once and runs one transform or two at a time.
 //
 // A cpair holds the same element of two independent transforms, component-wise: x = the two
-// real parts, y = the two imaginary parts.  Every operation is then one sm_100 paired FP32
-// instruction (add/mul/fma .f32x2) and needs no exchange between the halves: a rotation by i
-// is a renaming of registers, as for a single value.  (Packing the two components of one value
-// instead needs register moves for every rotation and twiddle, and measured slower.)  A paired
+// real parts, y = the two imaginary parts.  No operation needs an exchange between the halves: a
+// rotation by i is a renaming of registers, as for a single value.  (Packing the two components of
+// one value instead needs register moves for every rotation and twiddle, and measured slower.)  Sums
+// and differences are written as one sm_100 paired FP32 instruction (add.f32x2); products, whose
+// second factor is one value for both halves, as two scalar ones: a paired product would first copy
+// that factor into both halves of a register pair (288 against 282 us for a 64-template pass).  A paired
 // instruction takes two cycles of the FP32 pipe but one issue slot, so the pair leaves the other
 // slots to the shared-memory exchanges and addresses, and one twiddle, image value and address
 // serves two transforms.  Measured on B200: a radix-16 pass with its twiddles takes 303

@@ -233,8 +233,8 @@ __device__ __forceinline__ float2 dif_input(const float2 (&x)[R], int n1, int k2
     return k2 == 0 ? y : cmul(y, ld_tw(twr + n1 * k2));
 }
 
-// The radix-3 form of dif_input with its three inputs as scalars (the form the 1536-point
-// fused column pass was tuned with; the array form cost that kernel a register).
+// The radix-3 form of dif_input with its three inputs as scalars (the array form costs
+// the fused column pass a register).
 template <int P>
 __device__ __forceinline__ float2 dif_input3(float2 x0, float2 x1, float2 x2, int n1, int k2,
                                              const float2* __restrict__ tw3) {

@@ -491,8 +491,8 @@ struct BlockFft {
             constexpr int M = 16 / R;
             const float2* __restrict__ t = tw + S::TW_REM;
             // W_N^(r (j + T m)) = W_N^(r j) W_16^(r m): R-1 loads, the rest are constant turns
-            // (fewer L1 wavefronts, the binding unit of the row passes; measured on B200:
-            // C2R 2.97 instead of 3.10 us per template at 1536 points)
+            // (fewer L1 wavefronts, the binding unit of the row passes; measured on B200 with the
+            // C2R that ran 1536 points as three of these: 2.97 instead of 3.10 us per template)
             float2 wj[R];
 #pragma unroll
             for (int r = 1; r < R; r++) wj[r] = ld_tw(t + (r - 1) * (N / R) + j);

@@ -17,7 +17,7 @@
 // whose synchronisation is __syncwarp().  Length 1536 as 24 x 64 moves 8 x N values through
 // shared memory per forward-inverse pair and reads its input once; as three 512-point FFTs of
 // 16-value threads and a radix-3 step it moved 10 x N and read the input three times, and the
-// shared-memory path (75 % busy, 333 us per 64-template launch against 266) was what bound the
+// shared-memory path (75 % busy, 333 us per 64-template launch against 265) was what bound the
 // pass.
 //
 // C = float2 runs one transform, C = cpair two at a time (cpair.cuh).

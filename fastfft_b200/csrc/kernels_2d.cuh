@@ -115,7 +115,7 @@ using RowGroup = FftGroup<N, FPB, false, kBlockPad<N, FPB>>;
 // in reverse order, so that each pass starts on the data its predecessor wrote last).
 // Templates per launch of the batched passes (grid.y).  Up to 64: more templates per launch
 // mean more blocks per launch and a shorter partly empty last wave in all three passes
-// (measured on B200 at 1536^2: 13.8, 12.1 and 11.5 us per template at 16, 32 and 64).
+// (measured on B200, 64 templates at 1536^2: 577, 549 and 519 us at 16, 32 and 64 per launch).
 constexpr int kMaxBatch = 64;
 
 struct RowFwdArgs {
@@ -269,7 +269,8 @@ struct ColArgs {
 // the 256-point passes also read four columns per bank in the coalesced store.  The 4096-point passes (one column per block) likewise run better
 // with one buffer and four blocks, three for the correlation (24 - 32 instead of 16 - 24 warps per
 // SM; a forward transform of 4096^2 68.0 instead of 71.7 us, a single correlation 54.9 instead of
-// 56.4).
+// 56.4).  At four blocks (64 registers) the compiler spills 12 - 20 bytes per thread up to 256
+// points, 36 - 60 at 512 to 2048 and 28 at 4096; the figures include them.
 template <int N, int MODE, int FPB>
 struct ColGroup {
     static constexpr bool kMany = (FPB > 1 && MODE != COL_XCORR) || N == 4096;

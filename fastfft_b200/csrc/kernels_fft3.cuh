@@ -58,8 +58,7 @@ r2c3_rows_kernel(RowFwdArgs a) {
     const int j = t - k2 * TP;
     G g(smem, f, k2);
     // batch entries in reverse order: the fused column pass that follows starts with entry 0,
-    // whose rows are then the last written and still in L2 (measured on B200 with the C2R's
-    // reversal: 9.76 instead of 9.79 us per template at 1536^2, 2.91 instead of 2.96 at 768^2)
+    // whose rows are then the last written and still in L2
     const int gb = gridDim.y - 1 - blockIdx.y;
     const int n_rows = a.rows_g[gb] > 0 ? a.rows_g[gb] : a.n_rows;
     const int L = a.L_g[gb] > 0 ? a.L_g[gb] : a.L;
@@ -118,9 +117,10 @@ r2c3_rows_kernel(RowFwdArgs a) {
 // Row C2R (inverse), optional fused peak search
 // ---------------------------------------------------------------------------
 // The C2R gathers its input from L2/HBM with all of a thread's loads in flight at once, so it
-// gains from a third resident block per SM (56 registers; measured on B200 with this form of the
-// 1536-point pass: 4.2 instead of 4.6 us per template; at 4 blocks, 40 registers and spills, 3.96
-// against 2.81 at 3); the R2C does not (2.086 against 2.093), and keeps two.
+// gains from a third resident block per SM (56 registers); a fourth (40 registers) spills.  The R2C
+// gains nothing from a third, and keeps two.  (Measured on B200 at 1536 points, per template: C2R 4.2
+// instead of 4.6 us with three, 3.96 against 2.81 with four; R2C 2.086 against 2.093.  That length
+// has since moved to the split block FFT; the others kept the budgets.)
 #ifndef FFB_C2R3_MIN_BLOCKS
 #define FFB_C2R3_MIN_BLOCKS 3
 #endif

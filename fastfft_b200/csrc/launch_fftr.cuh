@@ -94,7 +94,7 @@ static cudaError_t r2c_split_impl(const RowFwdArgs& a0, cudaStream_t st) {
 }
 template <int N, class OutT>
 static cudaError_t c2r_split_impl(const RowInvArgs& a0, cudaStream_t st) {
-        constexpr int FPB = split_rows_fpb<N>(), MINB = N == 1536 ? 3 : 4;
+    constexpr int FPB = split_rows_fpb<N>(), MINB = N == 1536 ? 3 : 4;
     using SR = SplitRows<N, FPB>;
     RowInvArgs a = a0;
     cudaError_t e = split_twiddles_for(N, &a.tw);

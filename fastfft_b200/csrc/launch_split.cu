@@ -27,7 +27,7 @@ static bool pair_fits(int L) {
 // launch; "before": the radix-16 forms xcorr_cols_kernel / xcorr3_cols_kernel, which keep the
 // other lengths):
 //   length (template, window, templates)   before   single value   pair
-//   1536 (384, 1024, 64)                     333    288 (2 x 4)    266 (2 x 3), 284 (3 x 2)
+//   1536 (384, 1024, 64)                     333    288 (2 x 4)    265 (2 x 3), 284 (3 x 2)
 //   1536 (384, 1024, 12)                      85     65 (2 x 4)     67 (3 x 2)
 //   1536 (384, 1024, 1)                     17.2   13.9 (1 x 8)   18.3 (1 x 6)
 //   768  (256, 512, 64)                       90     80 (4 x 4)     80 (4 x 3)
@@ -42,16 +42,18 @@ static bool pair_fits(int L) {
 // rows at 1536 and 1600 at 2048.  Above, two blocks (8 warps) are the slower form (us per launch, pair
 // / single, same length and launch size, the window filling the length; both are flat on either
 // side of the line):
-//   1536, L = 448:  80.6 / 82.3 (16 templates)  153.8 / 154.5 (32)  282 / 295 (64)
-//   1536, L = 449:  91.7 / 82.2                 171.1 / 155.0       325 / 295
-//   1536, L = 1000: 92.5 / 86.0                 173.6 / 161.7       330 / 308
-//   2048, L = 1000: 135.2 / 138.3 (16)          258 / 264 (32)
-//   2048, L = 1590: 144.5 / 142.0               277 / 273
-//   2048, L = 1610: 159.2 / 142.7               305 / 273
+//   1536, L = 448:  79.3 / 82.0 (16 templates)  151.9 / 154.2 (32)  277 / 294 (64)
+//   1536, L = 449:  89.2 / 81.9                 167.4 / 154.8       316 / 295
+//   1536, L = 1000: 89.5 / 86.0                 166.8 / 161.7       317 / 308
+//   2048, L = 1000: 135.6 / 138.9 (16)          259 / 265 (32)
+//   2048, L = 1590: 145.7 / 142.6               278 / 273
+//   2048, L = 1610: 159.4 / 143.0               306 / 273
 // Fewer than four templates take blocks of one group, so that no group
-// idles.  At 1536 the pair's launch keeps the FP32 pipe 53 %, the shared-memory path 65 % and the
-// issue slots 57 % busy at 3 warps per scheduler: bound by latency at that occupancy (before: 48,
-// 75 and 71 %).  Both forms give the same bits (cpair.cuh), so the choice does not show in results.
+// idles.  At 1536 the pair's launch keeps the FP32 pipe 56 %, the shared-memory path 67 % and the
+// issue slots 60 % busy at 3 warps per scheduler: bound by latency at that occupancy (before: 48,
+// 75 and 71 %).  Spills per thread at 128 registers: 76 bytes at 1536 (2 x 4; 36 at 1 x 8), 32 at 2048,
+// 20 at 768 (4 x 4); the pairs have none.  Both forms give the same bits (cpair.cuh), so the choice
+// does not show in results.
 cudaError_t launch_xcorr_split(int n, const XcorrColArgs& a0, cudaStream_t st) {
     XcorrColArgs a = a0;
     if (a.n_batch < 1 || a.n_batch > kMaxBatch || a.n_cols < 1 || a.L < 1 || a.L > n) return cudaErrorInvalidValue;

@@ -27,9 +27,9 @@
 
 using namespace ffb;
 
-// Templates per block of the fused column pass where xcorr_tpb below makes no choice of its own (0:
-// the whole launch's group).  Fewer per block give more blocks and a shorter last, partly empty wave;
-// the image column is then staged by more blocks, from L2.
+// Templates per block of the fused column pass: a value other than 8 takes the place of xcorr_tpb's
+// choices below (0: the whole launch's group).  Fewer per block give more blocks and a shorter last,
+// partly empty wave; the image column is then staged by more blocks, from L2.
 #ifndef FFB_XCORR_TPB
 #define FFB_XCORR_TPB 8
 #endif
